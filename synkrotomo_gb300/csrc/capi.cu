@@ -286,6 +286,12 @@ int valid_split(int s) { return s == 1 || s == 2 || s == 4 || s == 8; }
 //   N=2048 / 1 slice even); batches of several problems keep the persistent
 //   kernel there.
 constexpr double kSmallWork = 6.0e7;
+// - a stack of at least two slices (deltarho 1) runs on the interleaved-slice
+//   kernels from kSmallStack on, where they pass the generic phases: us per
+//   iteration, generic / interleaved, N=128, 128 angles, 4 slices (2.0e7) 43 /
+//   65; N=64, 64 angles, 32 slices (2.0e7) 48 / 53; N=96, 90 angles, 16 slices
+//   (3.2e7) 70 / 66; N=512, 30 angles, 2 slices (3.8e7) 99 / 67.
+constexpr double kSmallStack = 2.8e7;
 
 int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double tol, int grid_blocks,
                void *staging = nullptr) {
@@ -329,9 +335,13 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
     const bool split = grid_blocks == -1 || (grid_blocks == 0 && !staging && (nprob == 1 || work <= kSmallWork));
     int fpg = 0, bpg = 0;
     if (split && !sirt_phase_grids(&fpg, &bpg)) return fail(ctx, SYNK_ECUDA, "SIRT phase kernels cannot be resident");
+    // a stack of slices: both phases on interleaved slices, the geometry evaluated once per group of them
+    const bool fits = split && nprob == 1 && in[0].nslices <= 65535 && (in[0].a + 31) / 32 + 2 <= 65535;
+    const bool slices = fits && in[0].nslices >= 2 && work > kSmallStack && in[0].deltarho == 1.0f &&
+                        slices_fit(make_geom(in[0].a, in[0].rhozero, in[0].deltarho, in[0].numrhos, in[0].size,
+                                             nullptr));
     // one large problem: the split engine's forward phase on the projector's own grid
-    const bool stack = split && nprob == 1 && work > kSmallWork && in[0].nslices <= 65535 &&
-                       (in[0].a + 31) / 32 + 2 <= 65535;
+    const bool stack = slices || (fits && work > kSmallWork);
     // the work splits fill the warps of the engine that runs the phases
     const long long fp_warps = split ? (long long)fpg * 8 : resident_warps;
     const long long bp_warps = split ? (long long)bpg * 8 : resident_warps;
@@ -375,9 +385,12 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         SYNK_CUDA(sc.get(&gcnt, 4), "cudaMallocAsync");
         SYNK_CUDA(sc.get(&R, pr), "cudaMallocAsync(R)");
         SYNK_CUDA(sc.get(&C, n), "cudaMallocAsync(C)");
-        SYNK_CUDA(sc.get(&xpad, np * q.nslices), "cudaMallocAsync(padded image)");
-        SYNK_CUDA(sc.get(&xTpad, np * q.nslices), "cudaMallocAsync(padded transposed image)");
-        SYNK_CUDA(sc.get(&rr, pr * q.nslices), "cudaMallocAsync(residual)");
+        // slices: xpad, xTpad and rr hold interleaved slice groups
+        const size_t npx = slices ? slices_floats(np, q.nslices) : np * q.nslices;
+        const size_t nrr = slices ? slices_floats(pr, q.nslices) : pr * q.nslices;
+        SYNK_CUDA(sc.get(&xpad, npx), "cudaMallocAsync(padded image)");
+        SYNK_CUDA(sc.get(&xTpad, npx), "cudaMallocAsync(padded transposed image)");
+        SYNK_CUDA(sc.get(&rr, nrr), "cudaMallocAsync(residual)");
         SYNK_CUDA(sc.get(&res2, K * q.nslices), "cudaMallocAsync");
         SYNK_CUDA(sc.get(&b2, (size_t)q.nslices), "cudaMallocAsync");
         SYNK_CUDA(sc.get(&stop_iter, (size_t)q.nslices), "cudaMallocAsync");
@@ -389,7 +402,7 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         // the backprojection-grid backward phase (one large problem, every
         // window of its 64-row tiles in range) reads rr as detector pairs
         float *rrp = nullptr;
-        if (stack && bp_windows_in_range(h.P, 64)) {
+        if (stack && !slices && bp_windows_in_range(h.P, 64)) {
             SYNK_CUDA(sc.get(&rrp, 2 * pr * q.nslices), "cudaMallocAsync(residual pairs)");
             SYNK_CUDA(cudaMemsetAsync(rrp, 0, sizeof(float) * 2 * pr * q.nslices, st), "memset");
         }
@@ -398,8 +411,14 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         SYNK_CUDA(launch_normalisers(h.P, R, C, graze, glen, goff, graze_tmp, glen_tmp, gcnt, graze_capc, st),
                   "normaliser kernels");
         // the listed rays' entries stay zero (their terms go to the corner pixels)
-        SYNK_CUDA(cudaMemsetAsync(rr, 0, sizeof(float) * pr * q.nslices, st), "memset");
-        SYNK_CUDA(launch_pad(q.out, xpad, xTpad, q.size, q.nslices, st), "pad kernel");
+        SYNK_CUDA(cudaMemsetAsync(rr, 0, sizeof(float) * nrr, st), "memset");
+        if (slices) {
+            SYNK_CUDA(cudaMemsetAsync(xpad, 0, sizeof(float) * npx, st), "memset");
+            SYNK_CUDA(cudaMemsetAsync(xTpad, 0, sizeof(float) * npx, st), "memset");
+            if (q.image) SYNK_CUDA(launch_slices_load(q.out, xpad, xTpad, q.size, q.nslices, st), "load kernel");
+        } else {
+            SYNK_CUDA(launch_pad(q.out, xpad, xTpad, q.size, q.nslices, st), "pad kernel");
+        }
         SYNK_CUDA(launch_sumsq(q.projections, pr, q.nslices, b2, st), "norm kernel");
         h.R = R;
         h.graze = graze;
@@ -420,7 +439,7 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         h.nslices = q.nslices;
         h.iterations = q.iterations;
         // warp tasks per phase: one detector x 32 angles (FP), one 32-column x 4-row strip (BP)
-        const long long fp_tasks = (long long)q.nslices * q.numrhos * ((q.a + 31) / 32);
+        const long long fp_tasks = (long long)(slices ? (q.nslices + 3) / 4 : q.nslices) * q.numrhos * ((q.a + 31) / 32);
         const long long bp_tasks = (long long)q.nslices * ((q.size + 3) / 4) * ((q.size + 31) / 32);
         const long long fp_share = nprob > 1 ? fp_warps / nprob + 1 : fp_warps;
         const long long bp_share = nprob > 1 ? bp_warps / nprob + 1 : bp_warps;
@@ -504,10 +523,14 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         const bool can_poll = sp.tol2 > 0.0 && !staging && cap == cudaStreamCaptureStatusNone;
         int poll_slot = 0, poll_prev = -1;
         for (int it = 0; it <= max_iter; ++it) {
-            if (stack) SYNK_CUDA(launch_sirt_fp_stack(host[0], it, sp.tol2, sp.record_final, st), "SIRT forward phase");
+            if (slices)
+                SYNK_CUDA(launch_sirt_fp_slices(host[0], it, sp.tol2, sp.record_final, sp.tol2 > 0.0 || want_res, st),
+                          "SIRT forward phase");
+            else if (stack) SYNK_CUDA(launch_sirt_fp_stack(host[0], it, sp.tol2, sp.record_final, st), "SIRT forward phase");
             else SYNK_CUDA(launch_sirt_fp_phase(sp, it, fpg, st), "SIRT forward phase");
             if (it == max_iter) break;
-            if (host[0].rrp) SYNK_CUDA(launch_sirt_bp_stack(host[0], it, sp.tol2, active, st), "SIRT backward phase");
+            if (slices) SYNK_CUDA(launch_sirt_bp_slices(host[0], it, sp.tol2, active, st), "SIRT backward phase");
+            else if (host[0].rrp) SYNK_CUDA(launch_sirt_bp_stack(host[0], it, sp.tol2, active, st), "SIRT backward phase");
             else SYNK_CUDA(launch_sirt_bp_phase(sp, it, active, bpg, st), "SIRT backward phase");
             // Every 16 iterations the count of slices still updating is copied
             // to pinned memory behind the backward phase, and the host waits
@@ -534,7 +557,9 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         SYNK_CUDA(launch_sirt_persistent(sp, grid, st), "persistent SIRT kernel");
     }
     for (int i = 0; i < nprob; ++i)
-        SYNK_CUDA(launch_unpad(host[i].xpad, in[i].out, in[i].size, in[i].nslices, st), "unpad kernel");
+        SYNK_CUDA(slices ? launch_slices_store(host[i].xpad, in[i].out, in[i].size, in[i].nslices, st)
+                         : launch_unpad(host[i].xpad, in[i].out, in[i].size, in[i].nslices, st),
+                  "unpad kernel");
     SYNK_CUDA(launch_sirt_finalize(dprobs, nprob, max_slices, sp.record_final, st), "finalize kernel");
     return SYNK_OK;
 }

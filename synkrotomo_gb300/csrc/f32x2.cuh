@@ -1,0 +1,47 @@
+// Packed pairs of float32 (the sm_100 family's f32x2 instructions): one
+// instruction issues the operation for both halves.  Each half rounds exactly
+// as the scalar instruction.  On GB300 a packed multiply-add takes the FMA pipe for two
+// cycles (two per clock and SM measured, four scalar ones), so packing saves
+// issue slots, not FMA-pipe time.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace synk {
+
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 pk2(float lo, float hi) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ f32x2 pk2(float2 v) { return pk2(v.x, v.y); }
+__device__ __forceinline__ float2 unpk2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2_rd(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2_ru(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rp.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+}  // namespace synk

@@ -29,6 +29,7 @@
 #include "sirt_internal.cuh"
 #include "fp_tile.cuh"
 #include "bp_tile.cuh"
+#include "sirt_device.cuh"
 
 namespace synk {
 
@@ -84,12 +85,6 @@ __device__ bool grid_barrier(unsigned *bar, unsigned nblocks, int *status, unsig
     return *s_flag != 0;
 }
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
-
 struct SirtShared {
     BpStage st;
     float red[8][33];
@@ -101,26 +96,11 @@ struct SirtShared {
     int any;
 };
 
-__device__ __forceinline__ int stop_of(const SirtProblem &q, int s) {
-    return *(volatile const int *)(q.stop_iter + s);
-}
-__device__ __forceinline__ double res2_of(const SirtProblem &q, int s, int it) {
-    return *(volatile const double *)(q.res2 + (size_t)s * (q.iterations + 1) + it);
-}
-
 // FP of iteration it is needed when the slice has not stopped before it and
 // it is at most the problem's last update (the final FP only measures).
 __device__ __forceinline__ bool fp_needed(const SirtParams &p, const SirtProblem &q, int s, int it) {
     if (it > q.iterations || (it == q.iterations && !p.record_final)) return false;
     return !(p.tol2 > 0.0 && stop_of(q, s) < it);
-}
-// BP (the update) of iteration it: the slice is below its count and neither
-// stopped before nor converged at x_it.
-__device__ __forceinline__ bool bp_needed(double tol2, const SirtProblem &q, int s, int it) {
-    if (it >= q.iterations) return false;
-    if (tol2 <= 0.0) return true;
-    if (stop_of(q, s) < it) return false;
-    return !(res2_of(q, s, it) <= tol2 * q.b2[s]);
 }
 __device__ __forceinline__ bool bp_needed(const SirtParams &p, const SirtProblem &q, int s, int it) {
     return bp_needed(p.tol2, q, s, it);
@@ -168,9 +148,6 @@ __device__ __forceinline__ double residual(const SirtProblem &q, int s, int k, i
     return (double)e * (double)e;
 }
 
-// Number of listed corner-clipping rays of a problem.
-__device__ __forceinline__ int graze_count(const SirtProblem &q) { return __ldg(q.goff + 4); }
-
 // Listed corner-clipping ray gidx (flat order: corner by corner) of slice s,
 // one warp; returns e^2 in lane 0.  The forward value comes from the
 // reference's row expressions over the rows the ray can touch (only the
@@ -200,20 +177,6 @@ __device__ __forceinline__ double graze_ray(const SirtProblem &q, int s, int gid
         e2 = (double)e * (double)e;
     }
     return e2;
-}
-
-// Backprojection terms of the listed rays that clip corner `corner` of slice
-// s, summed by the calling warp (lanes over the list, combined in a fixed
-// order); every lane returns the sum.
-__device__ __forceinline__ float corner_terms_warp(const SirtProblem &q, int s, int corner) {
-    const int lane = threadIdx.x & 31;
-    const int n = __ldg(q.goff + corner + 1) - __ldg(q.goff + corner);
-    const float *t = q.gcontrib + (size_t)s * 4 * q.graze_capc + (size_t)corner * q.graze_capc;
-    float acc = 0.0f;
-    for (int i = lane; i < n; i += 32) acc = __fadd_rn(acc, t[i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
-    return acc;
 }
 
 // Adds the block's e^2 of (problem q, slice) to its residual sum: every lane

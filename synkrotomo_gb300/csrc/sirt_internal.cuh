@@ -69,6 +69,15 @@ cudaError_t launch_sirt_fp_stack(const SirtProblem &q, int it, double tol2, int 
 // backward phase of the split engine for one problem on the backprojector's tile grid (needs q.rrp and every
 // detector window of its 64-row tiles inside the sinogram); block (0,0,0) applies the stopping rule into *active
 cudaError_t launch_sirt_bp_stack(const SirtProblem &q, int it, double tol2, int *active, cudaStream_t stream);
+// slice groups (sirt_slices.cu): both phases of a stack of at least two slices with deltarho 1 on interleaved
+// slices (xpad, xTpad and rr of the problem hold the groups); want_e2: the residual sums are read (tol or history)
+size_t slices_floats(size_t per_slice, int nslices);   // floats of a group buffer with per_slice entries a slice
+bool slices_fit(const ProbGeom &P);                     // 32-bit offsets suffice
+cudaError_t launch_slices_load(const float *x, float *xs, float *xTs, int N, int nslices, cudaStream_t stream);
+cudaError_t launch_slices_store(float *xs, float *x, int N, int nslices, cudaStream_t stream);
+cudaError_t launch_sirt_fp_slices(const SirtProblem &q, int it, double tol2, int record_final, int want_e2,
+                                  cudaStream_t stream);
+cudaError_t launch_sirt_bp_slices(const SirtProblem &q, int it, double tol2, int *active, cudaStream_t stream);
 cudaError_t launch_sirt_finalize(SirtProblem *probs, int nprob, int max_slices, int record_final,
                                  cudaStream_t stream);
 

@@ -215,6 +215,33 @@ __device__ __forceinline__ float fp_row_exact(const float *__restrict__ img, int
     return __fadd_rn(bot, top);
 }
 
+// The same row's two pixels and lengths, for kernels that apply them to several
+// slices (fp_row_exact's expressions).
+struct ExactRow {
+    int xpb, xpt;        // centred columns of the two pixels
+    float lbot, ltop;    // lengths in them
+    bool botin, topin;   // inside the image (topin false for a one-pixel row)
+};
+__device__ __forceinline__ ExactRow fp_row_exact_terms(int half, float slope, float intercept, float lbase, int i) {
+    ExactRow e;
+    const float xbot = __fadd_rn(__fmul_rn((float)i, slope), intercept);
+    const float xtop = __fadd_rn(xbot, slope);
+    e.xpb = (int)floorf(xbot);
+    e.xpt = (int)floorf(xtop);
+    const bool single = e.xpb == e.xpt;
+    e.botin = e.xpb >= -half && e.xpb < half;
+    e.topin = (!single) && e.xpt >= -half && e.xpt < half;
+    e.lbot = lbase;
+    e.ltop = 0.0f;
+    if (!single) {
+        const float xpmax = (float)max(e.xpb, e.xpt);
+        const float xdiff = __fsub_rn(xtop, xbot);
+        e.lbot = __fmul_rn(__fdiv_rn(__fsub_rn(xpmax, xbot), xdiff), lbase);
+        e.ltop = __fmul_rn(__fdiv_rn(__fsub_rn(xtop, xpmax), xdiff), lbase);
+    }
+    return e;
+}
+
 // All rows of a near-axis line, in the reference's order.
 template <bool ONES>
 __device__ __forceinline__ void fp_rows_exact(const float *__restrict__ img, int stride, int half, float slope,
@@ -312,6 +339,40 @@ __device__ __forceinline__ float bp_angle(const ProbGeom &P, const AngleGeom &g,
         if (det >= 0 && det < D) acc = __fadd_rn(acc, __fmul_rn(l, ONES ? 1.0f : __ldg(sino_row + det)));
     }
     return acc;
+}
+
+// bp_angle's near-axis branch for kernels that apply a weight to several
+// slices: the same expressions, calling f(detector, length) for every candidate
+// detector inside the sinogram, in the reference's order.
+template <class F>
+__device__ __forceinline__ void bp_exact_terms(const ProbGeom &P, const AngleGeom &g, int row, int col, F f) {
+    const int half = P.half;
+    const float xmin = (float)(g.flat ? row - half : col - half);
+    const float ymin = (float)(g.flat ? col - half : row - half);
+    const float fact = fact_f32();
+    const float cost = g.cost, sint = g.sint;
+    const float x = __fsub_rn(__fadd_rn(xmin, 0.5f), __fmul_rn(fact, cost));
+    const float y = __fsub_rn(__fadd_rn(ymin, 0.5f), __fmul_rn(fact, sint));
+    const float rho = __fadd_rn(__fmul_rn(cost, x), __fmul_rn(sint, y));
+    const float s = ceilf(__fdiv_rn(__fsub_rn(rho, P.rhozero), P.deltarho));
+    const float xbase = __fmul_rn(ymin, g.slope);
+    for (int i = 0; i < P.rpp; ++i) {
+        const float sprime = __fadd_rn(s, (float)i);
+        const float r = __fadd_rn(__fmul_rn(sprime, P.deltarho), P.rhozero);
+        const float xbot = __fadd_rn(xbase, __fdiv_rn(r, cost));
+        const float xtop = __fadd_rn(xbot, g.slope);
+        const float maxx = fmaxf(xbot, xtop), minx = fminf(xbot, xtop);
+        // intersect_fact (backprojection.fut:22-33)
+        const float lo = fmaxf(__fsub_rn(maxx, xmin), 0.0f);
+        const float hi = fmaxf(__fsub_rn(__fadd_rn(xmin, 1.0f), minx), 0.0f);
+        const float diff = __fsub_rn(maxx, minx);
+        const float inside = fminf(lo, hi);
+        // inside/0 is +inf in the reference, capped to 1 below
+        const float prop = inside == 0.0f ? 0.0f : (diff == 0.0f ? 1.0f : __fdiv_rn(inside, diff));
+        const float l = __fmul_rn(fminf(prop, 1.0f), g.lbase);
+        const int det = (int)sprime;
+        if (det >= 0 && det < P.D) f(det, l);
+    }
 }
 
 __device__ __forceinline__ AngleGeom load_geom(const AngleGeom *__restrict__ gt, int k) {
