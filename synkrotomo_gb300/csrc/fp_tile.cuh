@@ -10,7 +10,8 @@
 // walk takes the warp's union of the lanes' row ranges.  Two image layouts:
 //   fp_lane_ray_pair (standalone projector): pair images, entry i of a row =
 //     (pixel i-1, pixel i - pixel i-1) with zeros outside the image and a zero
-//     entry ending the row; one unconditional 8-byte gather per row step.
+//     entry ending the row; one unconditional 8-byte gather per row step, the
+//     arithmetic of two rows packed (f32x2.cuh).
 //   fp_lane_ray (SIRT, whose iterate is kept padded): row stride N+2, a zero
 //     column on each side, so one predicate covers both 4-byte gathers.
 // Per lane and row (forwardprojection.fut:31-56):
@@ -21,17 +22,18 @@
 // expressions (fp_exact in project.cu / the SIRT kernel).
 #pragma once
 
+#include "f32x2.cuh"
 #include "synk_internal.cuh"
 
 namespace synk {
 
 // Rows per partial sum of a ray before it enters the compensated (Neumaier)
 // total: plain float32 within a chunk, compensated across chunks.  Longer
-// chunks mean fewer compensation steps and a tighter row loop; measured at
-// N=2048 / 2048 angles, the standalone projector takes 4.54 / 4.34 / 4.22 /
-// 4.17 ms with 32 / 64 / 128 / 256 rows, and the SIRT slice stack (N=512,
-// 360 angles) 107.8 / 106.7 / 105.8 us per slice-iteration with 32 / 64 /
-// 128 (the last with 128-angle backprojection chunks).  A float32 partial
+// chunks mean fewer compensation steps and a tighter row loop; measured before
+// the packed walks at N=2048 / 2048 angles, the standalone projector took 4.54
+// / 4.34 / 4.22 / 4.17 ms with 32 / 64 / 128 / 256 rows, and the SIRT slice
+// stack (N=512, 360 angles) 107.8 / 106.7 / 105.8 us per slice-iteration with
+// 32 / 64 / 128.  A float32 partial
 // sum of n terms errs by at most (n - 1) * 2^-24 of the terms' absolute sum,
 // so 256 rows stay far inside the 1e-5 parity bar, and a 2048-row ray still
 // gets 8 compensated chunks.
@@ -157,59 +159,139 @@ __device__ __forceinline__ float fp_lane_ray(const ProbGeom &P, int k, int r, co
     return fp_lane_walk(P, L, img_pad);
 }
 
-// fp_lane_ray on a pair image: pair[j*(N+2) + i] = (pad(j, i), pad(j, i+1) -
-// pad(j, i)) for i in [0, N+1], where pad(j, i) = pixel (j, i-1) and 0 outside
-// [1, N]; entry N+1 of every row is (0, 0).  One 8-byte gather per row serves
-// both pixels of the row segment (v0 + t*(v1 - v0) is one FMA on the entry).
-// Its index comes from the bits of r = x + kMagic rounded down,
-// c + 1 = bits(r) - (kMagicBits - 1 - half), clamped as unsigned to N+1: a segment
-// left of column -1 wraps to a huge value and one right of N-1 exceeds N, and
-// both read the zero entry.  The loads are unconditional, so the rows of one
-// unrolled step issue their gathers back to back.
-__device__ __forceinline__ float fp_lane_ray_pair(const ProbGeom &P, int k, int r, const float2 *__restrict__ pair,
-                                                  int jb, int je) {
+// A warp's rays for the packed walks: the lane's line, the warp's union [J0, J1) of
+// the rows in which a lane's segment touches the image, and the warp's inner
+// rows [I0, I1) in which every lane's segment lies in columns [0, N): there
+// the gather index needs no clamp.  The inner bound keeps one pixel of slack on
+// each side (the zero columns), far above the rounding of x.  Lanes without a
+// ray (or whose ray misses the rows) walk column N/2 and return 0.
+struct WarpRay {
+    float x0, slope, ainv, lbase;
+    int J0, J1, I0, I1;
+    bool valid;
+};
+
+__device__ __forceinline__ WarpRay warp_ray(const ProbGeom &P, int k, int r, int jb, int je) {
     const AngleGeom g = load_geom(P.geom, k >= 0 ? k : 0);
     const float rho = __fadd_rn(P.rhozero, __fmul_rn((float)r, P.deltarho));    // forwardprojection.fut:28
     const float intercept = __fdiv_rn(rho, g.cost);                               // forwardprojection.fut:29
-    const float x0 = ray_x0(g, intercept);
+    WarpRay R;
+    R.x0 = ray_x0(g, intercept);
+    R.slope = g.slope;
+    R.ainv = g.ainv;
+    R.lbase = g.lbase;
     int j0 = 0, j1 = 0;
-    if (k >= 0 && !(fabsf(rho) > 0.75f * (float)P.N + 2.0f)) lane_rows(P, g, x0, j0, j1);
+    if (k >= 0 && !(fabsf(rho) > 0.75f * (float)P.N + 2.0f)) lane_rows(P, g, R.x0, j0, j1);
     j0 = max(j0, jb);
     j1 = min(j1, je);
-    if (j1 <= j0) { j0 = je; j1 = je; }
-    const int J0 = __reduce_min_sync(0xffffffffu, j0);
-    const int J1 = __reduce_max_sync(0xffffffffu, j1);
-    const float slope = g.slope, ainv = g.ainv;
-    const uintptr_t rowbytes = (uintptr_t)(P.N + 2) * 8u;
-    const unsigned zix = (unsigned)P.N + 1u;                   // the zero entry of a row
-    // bits(r) - okbase = c + 1 with c = floor(x) + half the pixel index
-    const unsigned okbase = (unsigned)kMagicBits - 1u - (unsigned)P.half;
-    const uintptr_t base = reinterpret_cast<uintptr_t>(pair);
-    const float x1 = x0 + slope, x2 = x0 + 2.0f * slope, x3 = x0 + 3.0f * slope;
-    float sum = 0.0f, comp = 0.0f;
-    auto row = [&](float x, uintptr_t rowb, float &part) {
-        const float rr = __fadd_rd(x, kMagic);
-        const float fl = __fsub_rn(rr, kMagic);
-        const float t = right_share(x, fl, ainv);
-        const unsigned ix = min((unsigned)__float_as_int(rr) - okbase, zix);
-        const float2 v = __ldg(reinterpret_cast<const float2 *>(rowb + (uintptr_t)ix * 8u));
-        part += fmaf(t, v.y, v.x);
-    };
-    for (int j = J0; j < J1;) {
-        const int jend = min(j + kPairCompRows, J1);
-        float part = 0.0f;
-        float jf = (float)(j - P.half);
-        uintptr_t rowb = base + (uintptr_t)j * rowbytes;
-        for (; j + 3 < jend; j += 4, jf += 4.0f, rowb += 4 * rowbytes) {
-            row(fmaf(jf, slope, x0), rowb, part);
-            row(fmaf(jf, slope, x1), rowb + rowbytes, part);
-            row(fmaf(jf, slope, x2), rowb + 2 * rowbytes, part);
-            row(fmaf(jf, slope, x3), rowb + 3 * rowbytes, part);
-        }
-        for (; j < jend; ++j, jf += 1.0f, rowb += rowbytes) row(fmaf(jf, slope, x0), rowb, part);
-        comp_add(sum, comp, part);
+    R.valid = j1 > j0;
+    int i0 = jb, i1 = je;
+    if (R.valid && !(fabsf(R.x0) < 1.0e6f && fabsf(R.slope) < 2.0f)) {
+        i0 = je;                            // no line (a non-finite angle): every row clamped
+        i1 = jb;
+    } else if (R.valid) {
+        // rows with -half <= x <= half - 1 (fast-path angles: |slope| >= 2^-12)
+        const float halff = (float)P.half;
+        const float ja = halff + (-halff - R.x0) / g.slope;
+        const float jz = halff + (halff - 1.0f - R.x0) / g.slope;
+        i0 = (int)fminf(fmaxf(fminf(ja, jz), -1.0f), (float)P.N) + 2;
+        i1 = (int)fmaxf(fminf(fmaxf(ja, jz), (float)P.N + 1.0f), 0.0f) - 1;
+    } else {
+        j0 = j1 = je;
+        R.x0 = 0.0f;
+        R.slope = 0.0f;
     }
-    return k >= 0 ? (sum + comp) * g.lbase : 0.0f;
+    R.J0 = __reduce_min_sync(0xffffffffu, j0);
+    R.J1 = __reduce_max_sync(0xffffffffu, j1);
+    i0 = __reduce_max_sync(0xffffffffu, i0);
+    i1 = __reduce_min_sync(0xffffffffu, i1);
+    R.I0 = min(max(i0, R.J0), R.J1);
+    R.I1 = min(max(i1, R.I0), R.J1);
+    return R;
+}
+
+// Ray sums on a pair image: entry i in [0, N+1] of row j is (pad(j, i), pad(j,
+// i+1) - pad(j, i)), where pad(j, i) = pixel (j, i-1) and 0 outside [1, N]; entry
+// N+1 of every row is (0, 0).  One 8-byte gather per row serves both pixels of
+// the row segment (v0 + t*(v1 - v0)).
+//
+// Rows go in packed pairs, four to a step.  The gather's byte offset comes from
+// the bits of r = x + kMagic rounded down, c + 1 = bits(r) - (kMagicBits - 1 -
+// half), clamped (as unsigned, to the zero entry N+1) only outside the warp's
+// inner rows.  `base` must be one address for the whole grid (the steep class's
+// image) and the frame image start `plane` bytes after it: with 32-bit offsets
+// from a uniform base a gather's address costs less than with a pointer chosen
+// per class (N=2048, 2048 angles: 3.06 ms against 3.37).  What is left is the
+// FMA pipe: nine of its cycles per step (packed adds and multiply-adds take two each).
+// All 32 lanes of the warp must call it.
+__device__ __forceinline__ float fp_lane_ray_pair(const ProbGeom &P, int k, int r, const char *__restrict__ base,
+                                                  unsigned plane, int jb, int je) {
+    const WarpRay R = warp_ray(P, k, r, jb, je);
+    const unsigned W = (unsigned)(P.N + 2) * 8u;                              // bytes of a row
+    const unsigned zix = (unsigned)P.N + 1u;
+    const unsigned okbase = (unsigned)kMagicBits - 1u - (unsigned)P.half;   // bits(r) - okbase = c + 1
+    const f32x2 sl2 = pk2(R.slope, R.slope), x02 = pk2(R.x0, R.x0);
+    const f32x2 mg2 = pk2(kMagic, kMagic), m1 = pk2(-1.0f, -1.0f), four2 = pk2(4.0f, 4.0f);
+    const float ainv = R.ainv, omv = __fsub_rn(1.0f, R.ainv);
+    float sum = 0.0f, comp = 0.0f;
+    auto rows = [&](int ja, int jz, bool clamp) {
+        for (int j = ja; j < jz;) {
+            const int jend = min(j + kPairCompRows, jz);
+            float pv = 0.0f, pd = 0.0f;
+            const float jf = (float)(j - P.half);
+            f32x2 ja2 = pk2(jf, jf + 1.0f), jb2 = pk2(jf + 2.0f, jf + 3.0f);
+            // byte offsets of four rows (mod 2^32), okbase folded in where unclamped
+            unsigned row0 = plane + (unsigned)j * W - (clamp ? 0u : okbase * 8u);
+            unsigned row1 = row0 + W, row2 = row0 + 2u * W, row3 = row0 + 3u * W;
+            auto split = [&](f32x2 j2, unsigned &ia, unsigned &ib, float &ta, float &tb) {
+                const f32x2 x = fma2(j2, sl2, x02);
+                const f32x2 rr = add2_rd(x, mg2);
+                const float2 f = unpk2(add2(x, fma2(rr, m1, mg2))), rv = unpk2(rr);      // x - floor(x)
+                ia = (unsigned)__float_as_int(rv.x);
+                ib = (unsigned)__float_as_int(rv.y);
+                if (clamp) {
+                    ia = min(ia - okbase, zix);
+                    ib = min(ib - okbase, zix);
+                }
+                ta = __saturatef(__fmaf_rn(f.x, ainv, omv));
+                tb = __saturatef(__fmaf_rn(f.y, ainv, omv));
+            };
+            auto ld = [&](unsigned off) { return __ldg(reinterpret_cast<const float2 *>(base + off)); };
+            auto add = [&](float2 v, float t) {
+                pv += v.x;
+                pd = fmaf(t, v.y, pd);
+            };
+            unsigned i0, i1, i2, i3;
+            float t0, t1, t2, t3;
+            for (; j + 3 < jend; j += 4) {
+                split(ja2, i0, i1, t0, t1);
+                split(jb2, i2, i3, t2, t3);
+                const float2 v0 = ld(i0 * 8u + row0), v1 = ld(i1 * 8u + row1), v2 = ld(i2 * 8u + row2),
+                             v3 = ld(i3 * 8u + row3);
+                add(v0, t0);
+                add(v1, t1);
+                add(v2, t2);
+                add(v3, t3);
+                row0 += 4u * W;
+                row1 += 4u * W;
+                row2 += 4u * W;
+                row3 += 4u * W;
+                ja2 = add2(ja2, four2);
+                jb2 = add2(jb2, four2);
+            }
+            for (; j < jend; ++j) {
+                split(ja2, i0, i1, t0, t1);
+                add(ld(i0 * 8u + row0), t0);
+                row0 += W;
+                ja2 = add2(ja2, pk2(1.0f, 1.0f));
+            }
+            comp_add(sum, comp, pv + pd);
+        }
+    };
+    rows(R.J0, R.I0, true);
+    rows(R.I0, R.I1, false);
+    rows(R.I1, R.J1, true);
+    return R.valid ? (sum + comp) * R.lbase : 0.0f;
 }
 
 // Ray of a near-axis angle k, the reference's own expressions

@@ -8,7 +8,7 @@
 //   forward:  fp_lane_kernel   8 detectors x 32 angles of one class per block
 //                              (4 angles x 8 detectors per warp; with row parts
 //                              one detector x 32 angles per warp)
-//             fp_det_kernel    fewer than 32 angles: one warp = 32 detectors of one angle
+//             fp_det_kernel    fewer than kFpDetAngles angles: one warp = 32 detectors of one angle
 //             fp_exact_kernel  near-axis angles, the reference's expressions
 //   backward: bp_tile_kernel   one block = 32 x 8*PIX pixels, PIX = 4 or 8 per thread, all angles
 //             bp_split_kernel  the same with the angles split over warps (images too small
@@ -337,18 +337,36 @@ cudaError_t launch_unpad(const float *xpad, float *x, int N, int nslices, cudaSt
 
 // ---- forward projection ---------------------------------------------------------
 
+// The two pair images of a projection as the kernels address them: 32-bit byte
+// offsets from one base, the transposed image `plane` bytes after it.  cls -1:
+// both classes; 0 / 1: the steep / flat angles only, their image at base (the two
+// images of the largest side, 16384, span more than 4 GB and take two
+// launches).  The kernels take the three as separate arguments: as members of a
+// struct argument the walk was 3 % slower.
+struct PairImages {
+    const char *base;
+    unsigned plane;
+    int cls;
+};
+
 // A block = 8 warps = 8/S detectors x S row parts (S = 1, 2, 4, 8; with S = 1
 // the block's 8 detectors x 32 angles are dealt 4 angles x 8 detectors per warp): with few
 // angles (sparse-view data) the rays are split over rows so that enough warps
 // are in flight; the S partial sums of a ray are added in a fixed order.
+// N=2048, 2048 angles: 4.18 -> 3.11 ms with the packed walk at 5 blocks per SM
+// (48 registers; 4 and 6 blocks were 5-8 % slower, and so were blocks of 512
+// and 1024 threads, whose L1 hit rate is higher: 79 and 86 % against 65).
 template <int S>
-__global__ void __launch_bounds__(256) fp_lane_kernel(ProbGeom P, AngleLists L, const float2 *__restrict__ xpair,
-                                                      const float2 *__restrict__ xTpair, float *__restrict__ sino) {
+__global__ void __launch_bounds__(256, 5) fp_lane_kernel(ProbGeom P, AngleLists L,
+                                                         const char *__restrict__ base, unsigned plane, int cls,
+                                                         float *__restrict__ sino) {
     __shared__ float red[8][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int grp = blockIdx.y;
     const int nsteep = __ldg(L.counts), nflat = __ldg(L.counts + 1);
     if (grp >= nsteep + nflat) return;              // block-uniform
+    const int flat = grp >= nsteep;
+    if (cls >= 0 && cls != flat) return;
     const int part = warp % S;
     int r, k;
     if (S == 1) {
@@ -364,7 +382,7 @@ __global__ void __launch_bounds__(256) fp_lane_kernel(ProbGeom P, AngleLists L, 
     }
     const int rr = r < P.D ? r : P.D - 1;          // keep every warp for the block reduction
     const int jb = part * P.N / S, je = (part + 1) * P.N / S;
-    float v = fp_lane_ray_pair(P, r < P.D ? k : -1, rr, grp < nsteep ? xpair : xTpair, jb, je);
+    float v = fp_lane_ray_pair(P, r < P.D ? k : -1, rr, base, flat ? plane : 0u, jb, je);
     if (S > 1) {
         red[warp][lane] = v;
         __syncthreads();
@@ -374,14 +392,15 @@ __global__ void __launch_bounds__(256) fp_lane_kernel(ProbGeom P, AngleLists L, 
     if (k >= 0 && r < P.D) sino[(size_t)k * P.D + r] = v;
 }
 
-// Fewer than 32 angles (sparse-view data): one warp = 32 consecutive detectors
-// of one angle, so no lane idles, and a block of 32 warps splits each ray into
-// S row parts (S up to 32, at least 16 rows a part) so that each warp's chain
-// of dependent gathers is short.  The per-ray arithmetic is fp_lane_kernel's
+// Fewer than kFpDetAngles angles (sparse-view data): one warp = 32 consecutive
+// detectors of one angle, so no lane idles and the lanes' row ranges nearly
+// agree, and a block of 32 warps splits each ray into S row parts (S up to 32, at
+// least 16 rows a part) so that each warp's chain of dependent gathers is short.  The per-ray arithmetic is fp_lane_kernel's
 // (fp_lane_ray_pair); the S partial sums are added in a fixed order.
 template <int S>
-__global__ void __launch_bounds__(1024, 2) fp_det_kernel(ProbGeom P, AngleLists L, const float2 *__restrict__ xpair,
-                                                      const float2 *__restrict__ xTpair, float *__restrict__ sino) {
+__global__ void __launch_bounds__(1024, 2) fp_det_kernel(ProbGeom P, AngleLists L,
+                                                         const char *__restrict__ base, unsigned plane, int cls,
+                                                         float *__restrict__ sino) {
     __shared__ float red[32][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int steep_slots = __ldg(L.counts) * 32;
@@ -390,11 +409,13 @@ __global__ void __launch_bounds__(1024, 2) fp_det_kernel(ProbGeom P, AngleLists 
     if (slot >= nslots) return;                       // block-uniform
     const int k = __ldg(L.order + slot);
     if (k < 0) return;                                // block-uniform: padding of a group
+    const int flat = slot >= steep_slots;
+    if (cls >= 0 && cls != flat) return;
     const int part = warp % S;
     const int r = (blockIdx.x * (32 / S) + warp / S) * 32 + lane;
     const int jb = part * P.N / S, je = (part + 1) * P.N / S;
     const bool in = r < P.D;
-    float v = fp_lane_ray_pair(P, in ? k : -1, in ? r : P.D - 1, slot < steep_slots ? xpair : xTpair, jb, je);
+    float v = fp_lane_ray_pair(P, in ? k : -1, in ? r : P.D - 1, base, flat ? plane : 0u, jb, je);
     if (S > 1) {
         red[warp][lane] = v;
         __syncthreads();
@@ -442,21 +463,28 @@ static int fp_row_split(long long warps) {
     return S;
 }
 
-cudaError_t launch_fp(const ProbGeom &P, const AngleLists &L, const float2 *xpair, const float2 *xTpair, float *sino,
-                      cudaStream_t stream) {
-    if (P.a < 32) {
-        // at most one group of each class: 64 angle slots; rows split to >= 16 a part
+// Angle count from which fp_lane_kernel runs.  Below it neighbouring angles lie so
+// far apart that a warp of 4 angles walks rows and reads lines its lanes share
+// little of.  Lane / detector kernel, us per call: N=2048, 64 angles 566 / 215;
+// N=1024, 95 angles 177 / 97; N=512, 95 angles 55 / 48; N=512, 180 angles 68 / 71;
+// N=2048, 256 angles 578 / 646.
+constexpr int kFpDetAngles = 160;
+
+static void launch_fp_rays(const ProbGeom &P, const AngleLists &L, const PairImages &X, float *sino,
+                           cudaStream_t stream) {
+    if (P.a < kFpDetAngles) {
+        // angle slots: the padded groups of 32 of both classes; rows split to >= 16 a part
         int S = 1;
         while (S < 32 && P.N / (2 * S) >= 16) S *= 2;
         const int dgroups = (P.D + 31) / 32;
-        const dim3 grid((dgroups + 32 / S - 1) / (32 / S), 64);
+        const dim3 grid((dgroups + 32 / S - 1) / (32 / S), ((P.a + 31) / 32 + 1) * 32);
         switch (S) {
-            case 1: fp_det_kernel<1><<<grid, 1024, 0, stream>>>(P, L, xpair, xTpair, sino); break;
-            case 2: fp_det_kernel<2><<<grid, 1024, 0, stream>>>(P, L, xpair, xTpair, sino); break;
-            case 4: fp_det_kernel<4><<<grid, 1024, 0, stream>>>(P, L, xpair, xTpair, sino); break;
-            case 8: fp_det_kernel<8><<<grid, 1024, 0, stream>>>(P, L, xpair, xTpair, sino); break;
-            case 16: fp_det_kernel<16><<<grid, 1024, 0, stream>>>(P, L, xpair, xTpair, sino); break;
-            default: fp_det_kernel<32><<<grid, 1024, 0, stream>>>(P, L, xpair, xTpair, sino); break;
+            case 1: fp_det_kernel<1><<<grid, 1024, 0, stream>>>(P, L, X.base, X.plane, X.cls, sino); break;
+            case 2: fp_det_kernel<2><<<grid, 1024, 0, stream>>>(P, L, X.base, X.plane, X.cls, sino); break;
+            case 4: fp_det_kernel<4><<<grid, 1024, 0, stream>>>(P, L, X.base, X.plane, X.cls, sino); break;
+            case 8: fp_det_kernel<8><<<grid, 1024, 0, stream>>>(P, L, X.base, X.plane, X.cls, sino); break;
+            case 16: fp_det_kernel<16><<<grid, 1024, 0, stream>>>(P, L, X.base, X.plane, X.cls, sino); break;
+            default: fp_det_kernel<32><<<grid, 1024, 0, stream>>>(P, L, X.base, X.plane, X.cls, sino); break;
         }
     } else {
         // groups of 32 angles: at most ceil(a/32) + 2 (the steep/flat split adds one partial group each)
@@ -464,11 +492,23 @@ cudaError_t launch_fp(const ProbGeom &P, const AngleLists &L, const float2 *xpai
         const int S = fp_row_split((long long)((P.a + 31) / 32) * P.D);
         const dim3 grid((P.D + 8 / S - 1) / (8 / S), gmax);
         switch (S) {
-            case 1: fp_lane_kernel<1><<<grid, 256, 0, stream>>>(P, L, xpair, xTpair, sino); break;
-            case 2: fp_lane_kernel<2><<<grid, 256, 0, stream>>>(P, L, xpair, xTpair, sino); break;
-            case 4: fp_lane_kernel<4><<<grid, 256, 0, stream>>>(P, L, xpair, xTpair, sino); break;
-            default: fp_lane_kernel<8><<<grid, 256, 0, stream>>>(P, L, xpair, xTpair, sino); break;
+            case 1: fp_lane_kernel<1><<<grid, 256, 0, stream>>>(P, L, X.base, X.plane, X.cls, sino); break;
+            case 2: fp_lane_kernel<2><<<grid, 256, 0, stream>>>(P, L, X.base, X.plane, X.cls, sino); break;
+            case 4: fp_lane_kernel<4><<<grid, 256, 0, stream>>>(P, L, X.base, X.plane, X.cls, sino); break;
+            default: fp_lane_kernel<8><<<grid, 256, 0, stream>>>(P, L, X.base, X.plane, X.cls, sino); break;
         }
+    }
+}
+
+cudaError_t launch_fp(const ProbGeom &P, const AngleLists &L, const float2 *xpair, const float2 *xTpair, float *sino,
+                      cudaStream_t stream) {
+    const char *b0 = reinterpret_cast<const char *>(xpair), *b1 = reinterpret_cast<const char *>(xTpair);
+    const unsigned long long gap = (unsigned long long)(b1 - b0);
+    if (b1 > b0 && gap + (unsigned long long)P.N * (P.N + 2) * 8ull < (1ull << 32)) {
+        launch_fp_rays(P, L, PairImages{b0, (unsigned)gap, -1}, sino, stream);
+    } else {
+        launch_fp_rays(P, L, PairImages{b0, 0u, 0}, sino, stream);
+        launch_fp_rays(P, L, PairImages{b1, 0u, 1}, sino, stream);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

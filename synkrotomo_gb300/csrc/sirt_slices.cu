@@ -59,64 +59,13 @@ __device__ __forceinline__ Vec<V> *group_ptr(float *base, int s0, size_t per_sli
 
 constexpr int kSlotsExact = 4;      // near-axis angle slots of the exact kernel (repeats loop)
 
-// A ray of the group kernels: the lane's line, the warp's union [J0, J1) of
-// the rows in which a lane's segment touches the image, and the warp's inner
-// rows [I0, I1) in which every lane's segment lies in columns [0, N): there
-// the gather index needs no clamp.  The inner bound keeps one pixel of slack on
-// each side (the zero columns), far above the rounding of x.  Lanes without a
-// ray (or whose ray misses the rows) walk column N/2 and return 0.
-struct GroupRay {
-    float x0, slope, ainv, lbase;
-    int J0, J1, I0, I1;
-    bool valid;
-};
-
-__device__ __forceinline__ GroupRay group_ray(const ProbGeom &P, int k, int r, int jb, int je) {
-    const AngleGeom g = load_geom(P.geom, k >= 0 ? k : 0);
-    const float rho = __fadd_rn(P.rhozero, __fmul_rn((float)r, P.deltarho));    // forwardprojection.fut:28
-    const float intercept = __fdiv_rn(rho, g.cost);                               // forwardprojection.fut:29
-    GroupRay R;
-    R.x0 = ray_x0(g, intercept);
-    R.slope = g.slope;
-    R.ainv = g.ainv;
-    R.lbase = g.lbase;
-    int j0 = 0, j1 = 0;
-    if (k >= 0 && !(fabsf(rho) > 0.75f * (float)P.N + 2.0f)) lane_rows(P, g, R.x0, j0, j1);
-    j0 = max(j0, jb);
-    j1 = min(j1, je);
-    R.valid = j1 > j0;
-    int i0 = jb, i1 = je;
-    if (R.valid && !(fabsf(R.x0) < 1.0e6f && fabsf(R.slope) < 2.0f)) {
-        i0 = je;                            // no line (a non-finite angle): every row clamped
-        i1 = jb;
-    } else if (R.valid) {
-        // rows with -half <= x <= half - 1 (fast-path angles: |slope| >= 2^-12)
-        const float halff = (float)P.half;
-        const float ja = halff + (-halff - R.x0) / g.slope;
-        const float jz = halff + (halff - 1.0f - R.x0) / g.slope;
-        i0 = (int)fminf(fmaxf(fminf(ja, jz), -1.0f), (float)P.N) + 2;
-        i1 = (int)fmaxf(fminf(fmaxf(ja, jz), (float)P.N + 1.0f), 0.0f) - 1;
-    } else {
-        j0 = j1 = je;
-        R.x0 = 0.0f;
-        R.slope = 0.0f;
-    }
-    R.J0 = __reduce_min_sync(0xffffffffu, j0);
-    R.J1 = __reduce_max_sync(0xffffffffu, j1);
-    i0 = __reduce_max_sync(0xffffffffu, i0);
-    i1 = __reduce_min_sync(0xffffffffu, i1);
-    R.I0 = min(max(i0, R.J0), R.J1);
-    R.I1 = min(max(i1, R.I0), R.J1);
-    return R;
-}
-
 // The ray's sums over rows [J0, J1) of the group's V slices on its padded
 // frame image (32-bit byte offsets: below 4 GB, checked by the host).  Per
 // row: x = (j - half)*slope + x0, c = floor(x) + half, t = share of column c+1,
 // sum += (1 - t)*v[c] + t*v[c+1].  Plain float32 over kSirtCompRows rows,
 // compensated across chunks.
 template <int V>
-__device__ __forceinline__ void group_walk(const ProbGeom &P, const GroupRay &R, const char *__restrict__ img,
+__device__ __forceinline__ void group_walk(const ProbGeom &P, const WarpRay &R, const char *__restrict__ img,
                                            float (&out)[V]) {
     constexpr unsigned EB = 4u * V;                                           // bytes of an entry
     const unsigned rowbytes = (unsigned)(P.N + 2) * EB;
@@ -260,7 +209,7 @@ __global__ void __launch_bounds__(256, 4) sirt_fp_slices_kernel(SirtProblem q, i
     const int jb = (int)((long long)part * q.P.N / S), je = (int)((long long)(part + 1) * q.P.N / S);
     const size_t np = (size_t)q.P.N * (q.P.N + 2);
     const Vec<V> *img = group_ptr<V>(grp < nsteep ? q.xpad : q.xTpad, s0, np);
-    const GroupRay R = group_ray(q.P, k, r, jb, je);
+    const WarpRay R = warp_ray(q.P, k, r, jb, je);
     float v[V];
     group_walk<V>(q.P, R, reinterpret_cast<const char *>(img), v);
     if (S > 1) {
