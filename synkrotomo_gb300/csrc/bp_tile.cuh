@@ -18,6 +18,7 @@
 // with zero weight and summed afterwards with the reference's own expressions.
 #pragma once
 
+#include "f32x2.cuh"
 #include "synk_internal.cuh"
 
 namespace synk {
@@ -66,16 +67,12 @@ __device__ __forceinline__ void bp_stage(const ProbGeom &P, int k0, BpStage &st)
 // SCALED: the sinogram rows of the staged (non-near-axis) angles are already
 // multiplied by their lbase (row_scale), which saves one multiply per
 // (pixel, angle); near-axis rows stay unscaled for bp_exact_angles.
-// UNR = 2 (4) walks the angles two (four) at a time, so that their gathers
-// are in flight together; the sums stay in angle order, bit for bit those of
-// UNR = 1.
-// PAIR (INRANGE only): sino holds detector pairs, entry s of row k =
-// (row[s], row[s+1]) at float offset 2*(k*D + s), so one 8-byte gather serves
-// both candidates (the same values, the same sums).
+// UNR = 2 walks the angles two at a time, so that their gathers are in flight
+// together; the sums stay in angle order, bit for bit those of UNR = 1.
 // Measured on GB300: SIRT at N=128 6.20 -> 5.88 ms (200 iterations; few warps
 // there hide the gathers' latency), the dense backprojector at N=2048 4.88 ->
 // 4.73 ms.
-template <int PIX, bool UNIT, bool INRANGE, bool SCALED, int UNR = 1, bool PAIR = false>
+template <int PIX, bool UNIT, bool INRANGE, bool SCALED, int UNR = 1>
 __device__ __forceinline__ void bp_chunk(const ProbGeom &P, const BpStage &st, int kc, int kend, int kphase,
                                          int kstride, const float *__restrict__ sino, float xc, float yc0,
                                          float ystep, float (&acc)[PIX]) {
@@ -85,12 +82,11 @@ __device__ __forceinline__ void bp_chunk(const ProbGeom &P, const BpStage &st, i
     const int nk = min(kBpChunk, kend - kc);
     const float zoff = -P.rz_c - fact;        // centred: |q| stays below ~N/sqrt(2) + 1
     // INRANGE gather base: row + zi - kMagicBits (the magic constant's bits folded in)
-    static_assert(!PAIR || INRANGE, "pair rows only on the in-range path");
-    const uintptr_t zoffb = (uintptr_t)(((intptr_t)P.zi - (intptr_t)kMagicBits) * (PAIR ? 8 : 4));
+    const uintptr_t zoffb = (uintptr_t)(((intptr_t)P.zi - (intptr_t)kMagicBits) * 4);
     auto angle = [&](int i) {
         const float4 g = st.cs[i];
         const float2 le = st.le[i];
-        const float *__restrict__ row = sino + (size_t)(kc + i) * D * (PAIR ? 2 : 1);
+        const float *__restrict__ row = sino + (size_t)(kc + i) * D;
         if constexpr (UNIT) {
             // q of pixel m from the angle's base value in one rounding
             // (fma(m, dq, q0)), not by repeated additions: those drift by up
@@ -109,17 +105,10 @@ __device__ __forceinline__ void bp_chunk(const ProbGeom &P, const BpStage &st, i
                 if constexpr (INRANGE) {
                     const float r = __fadd_ru(q, kMagic);
                     e = __fsub_rn(r, kMagic) - q;
-                    if constexpr (PAIR) {
-                        const float2 v = __ldg(reinterpret_cast<const float2 *>(
-                            rowb + (uintptr_t)(unsigned)__float_as_int(r) * 8u));
-                        v0 = v.x;
-                        v1 = v.y;
-                    } else {
-                        const float *p = reinterpret_cast<const float *>(
-                            rowb + (uintptr_t)(unsigned)__float_as_int(r) * 4u);
-                        v0 = __ldg(p);
-                        v1 = __ldg(p + 1);
-                    }
+                    const float *p = reinterpret_cast<const float *>(
+                        rowb + (uintptr_t)(unsigned)__float_as_int(r) * 4u);
+                    v0 = __ldg(p);
+                    v1 = __ldg(p + 1);
                 } else {
                     int s0;
                     e = ceil_magic(q, s0) - q;
@@ -153,19 +142,74 @@ __device__ __forceinline__ void bp_chunk(const ProbGeom &P, const BpStage &st, i
         }
     };
     int i = kphase;
-    if constexpr (UNR == 4)
-        for (; i + 3 * kstride < nk; i += 4 * kstride) {
-            angle(i);
-            angle(i + kstride);
-            angle(i + 2 * kstride);
-            angle(i + 3 * kstride);
-        }
     if constexpr (UNR >= 2)
         for (; i + kstride < nk; i += 2 * kstride) {
             angle(i);
             angle(i + kstride);
         }
     for (; i < nk; i += kstride) angle(i);
+}
+
+// The UNIT, INRANGE, SCALED path on detector pairs: entry s of row k is (row[s],
+// row[s+1]), so one 8-byte gather serves both candidates of a pixel and angle,
+// and one packed multiply-add (acc_0, acc_1) += (w0, w1) * (v0, v1).  Angles kc
+// .. of the staged chunk into out[m] (overwritten).  Two pixels' coordinates,
+// ceilings and fractions are computed at a time with packed instructions (the
+// halves round as the scalar ones), and a gather's address is a 32-bit offset
+// in the chunk's rows (a chunk of 256 in-range rows is below 4 GB): the 64-bit
+// wide multiply-add it replaces holds the FMA pipe for four to five cycles.
+// Two angles at a time with 80 registers (3 blocks per SM), N=2048, 2048 angles:
+// 4.05 -> 3.44 ms (one at a time 4.25; 64 registers 3.75; three with 128 registers
+// 3.62; the tile's segments staged in shared memory 3.88).
+template <int PIX>
+__device__ __forceinline__ void bp_chunk_pair(const ProbGeom &P, const BpStage &st, int kc,
+                                              const float2 *__restrict__ pairs, float xc, float yc0, float ystep,
+                                              float (&out)[PIX]) {
+    static_assert(PIX % 2 == 0, "pixels go in pairs");
+    const float fact = fact_f32();
+    const float zoff = -P.rz_c - fact;
+    const f32x2 mg2 = pk2(kMagic, kMagic), nmg2 = pk2(-kMagic, -kMagic), m1 = pk2(-1.0f, -1.0f);
+    const f32x2 nf2 = pk2(-fact, -fact);
+    const char *base = reinterpret_cast<const char *>(pairs + (size_t)kc * P.D);
+    const unsigned step = (unsigned)P.D * 8u;
+    // gather offset in the chunk = bits(r)*8 + rowoff (mod 2^32), bits(r) = kMagicBits + s0 - zi
+    unsigned rowoff = ((unsigned)P.zi - (unsigned)kMagicBits) * 8u;
+    const int nk = min(kBpChunk, P.a - kc);
+    f32x2 acc[PIX];
+#pragma unroll
+    for (int m = 0; m < PIX; ++m) acc[m] = pk2(0.0f, 0.0f);
+#pragma unroll 2
+    for (int i = 0; i < nk; ++i) {
+        const float4 g = st.cs[i];
+        const float c1 = st.le[i].y;
+        // q of pixel m from the angle's base value in one rounding (see bp_chunk)
+        const float q0 = fmaf(xc, g.x, fmaf(-yc0, g.y, zoff));
+        const float dq = -ystep * g.y;
+        const f32x2 q02 = pk2(q0, q0), dq2 = pk2(dq, dq);
+        float2 v[PIX], w[PIX];
+#pragma unroll
+        for (int h = 0; h < PIX / 2; ++h) {
+            const f32x2 q = fma2(pk2((float)(2 * h), (float)(2 * h + 1)), dq2, q02);
+            const f32x2 r = add2_ru(q, mg2);
+            const f32x2 e = fma2(q, m1, add2(r, nmg2));            // ceil(q) - q
+            const float2 ev = unpk2(e), dv = unpk2(add2(e, nf2)), rv = unpk2(r);
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                v[2 * h + o] = __ldg(reinterpret_cast<const float2 *>(
+                    base + ((unsigned)__float_as_int(o ? rv.y : rv.x) * 8u + rowoff)));
+                w[2 * h + o].x = __saturatef(fmaf(-fabsf(o ? dv.y : dv.x), g.w, g.z));
+                w[2 * h + o].y = __saturatef(fmaf(-(o ? ev.y : ev.x), g.w, c1));
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < PIX; ++m) acc[m] = fma2(pk2(w[m]), pk2(v[m]), acc[m]);
+        rowoff += step;
+    }
+#pragma unroll
+    for (int m = 0; m < PIX; ++m) {
+        const float2 t = unpk2(acc[m]);
+        out[m] = t.x + t.y;
+    }
 }
 
 // Factor of sinogram row k in a SCALED backprojection: lbase, or 1 for a

@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(256) row_scale_kernel(ProbGeom P, const float 
 }
 
 // pair[k][s] = (v[s], v[s+1]) with v = sino[k] * row_scale(k) and v[D] = 0:
-// the rows of a SCALED backprojection as detector pairs (bp_chunk's PAIR).
+// the rows of a SCALED backprojection as detector pairs (bp_chunk_pair).
 __global__ void __launch_bounds__(256) row_pair_kernel(ProbGeom P, const float *__restrict__ sino,
                                                        float2 *__restrict__ pair) {
     const int r = blockIdx.x * 256 + threadIdx.x;
@@ -562,11 +562,9 @@ constexpr int kBpManyAngles = 256;     // angle count from which the 8-pixel var
 
 // sino_s: the fast-path rows (scaled when SCALED, else sino itself); sino:
 // the unscaled rows read by the near-axis angles.
-// PAIR (the dense in-range path) walks the angles four at a time with 64
-// registers (4 blocks per SM): 4.52 -> 4.14 ms at N = 2048, 2048 angles
-// (two at a time with 48 registers and 5 blocks: 4.52; two with 64: 4.33).
+// PAIR (the dense in-range path): bp_chunk_pair.
 template <int kBpPix, bool UNIT, bool INRANGE, bool SCALED, bool PAIR = false>
-__global__ void __launch_bounds__(256, PAIR ? 4 : BpShape<kBpPix>::kMinBlocks) bp_tile_kernel(ProbGeom P, AngleLists L,
+__global__ void __launch_bounds__(256, PAIR ? 3 : BpShape<kBpPix>::kMinBlocks) bp_tile_kernel(ProbGeom P, AngleLists L,
                                                                    const float *__restrict__ sino_s,
                                                                    const float *__restrict__ sino,
                                                                    float *__restrict__ out) {
@@ -590,7 +588,9 @@ __global__ void __launch_bounds__(256, PAIR ? 4 : BpShape<kBpPix>::kMinBlocks) b
         float part[kBpPix];
 #pragma unroll
         for (int m = 0; m < kBpPix; ++m) part[m] = 0.0f;
-        bp_chunk<kBpPix, UNIT, INRANGE, SCALED, PAIR ? 4 : 2, PAIR>(P, st, kc, P.a, 0, 1, sino_s, xc, yc0, 8.0f, part);
+        if constexpr (PAIR)
+            bp_chunk_pair<kBpPix>(P, st, kc, reinterpret_cast<const float2 *>(sino_s), xc, yc0, 8.0f, part);
+        else bp_chunk<kBpPix, UNIT, INRANGE, SCALED, 2>(P, st, kc, P.a, 0, 1, sino_s, xc, yc0, 8.0f, part);
 #pragma unroll
         for (int m = 0; m < kBpPix; ++m) comp_add(sum[m], comp[m], part[m]);
     }

@@ -563,13 +563,13 @@ __global__ void __launch_bounds__(256, 4) sirt_bp_phase_kernel(SirtParams p, int
 // Backward phase of the split engine for one large problem (a slice stack)
 // on the standalone backprojector's grid: a block = 32 columns x 64 rows of
 // one slice (blockIdx.z), 8 rows per thread, the weighted residual read as
-// detector pairs (one 8-byte gather per pixel and angle), four angles at a
-// time, and the SIRT update x + C*bp (SIRT.fut:38-39) with both padded
-// copies of the iterate in the epilogue.  The angles are summed in the order
+// detector pairs (bp_chunk_pair), and the SIRT update x + C*bp
+// (SIRT.fut:38-39) with both padded copies of the iterate in the epilogue.  The angles are summed in the order
 // of bp_phase; a pixel's detector coordinate comes from its thread's first
 // row, so the iterates equal the generic phase's to rounding.  Block (0,0,0)
 // also applies the stopping rule of iteration it (sirt_bp_phase_kernel's rule).
-__global__ void __launch_bounds__(256, 4) sirt_bp_stack_kernel(SirtProblem q, int it, double tol2, int *active) {
+template <int MINB>
+__global__ void __launch_bounds__(256, MINB) sirt_bp_stack_kernel(SirtProblem q, int it, double tol2, int *active) {
     __shared__ BpStage st;
     __shared__ float tile[32][65];
     __shared__ int any;
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(256, 4) sirt_bp_stack_kernel(SirtProblem q, in
     const float xc = (float)(col - P.half) + 0.5f;
     const float yc0 = (float)(row0 - P.half) + 0.5f;
     const size_t pr = (size_t)P.a * P.D, np = (size_t)P.N * (P.N + 2);
-    const float *rows = q.rrp + (size_t)s * pr * 2;
+    const float2 *rows = reinterpret_cast<const float2 *>(q.rrp) + (size_t)s * pr;
     float sum[8], comp[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) sum[m] = comp[m] = 0.0f;
@@ -603,9 +603,7 @@ __global__ void __launch_bounds__(256, 4) sirt_bp_stack_kernel(SirtProblem q, in
         bp_stage(P, kc, st);
         __syncthreads();
         float part[8];
-#pragma unroll
-        for (int m = 0; m < 8; ++m) part[m] = 0.0f;
-        bp_chunk<8, true, true, true, 4, true>(P, st, kc, P.a, 0, 1, rows, xc, yc0, 8.0f, part);
+        bp_chunk_pair<8>(P, st, kc, rows, xc, yc0, 8.0f, part);
 #pragma unroll
         for (int m = 0; m < 8; ++m) comp_add(sum[m], comp[m], part[m]);
     }
@@ -651,7 +649,13 @@ __global__ void __launch_bounds__(256, 4) sirt_bp_stack_kernel(SirtProblem q, in
 
 cudaError_t launch_sirt_bp_stack(const SirtProblem &q, int it, double tol2, int *active, cudaStream_t stream) {
     const dim3 grid((q.P.N + 31) / 32, (q.P.N + 63) / 64, q.nslices);
-    sirt_bp_stack_kernel<<<grid, 256, 0, stream>>>(q, it, tol2, active);
+    // 80 registers and 3 blocks per SM run the walk faster (N=512, 360 angles, one
+    // slice: 277 us per iteration, 306 with 64 registers and 4 blocks; N=768, 720
+    // angles 727 / 780), except where they would need a second wave that 4 blocks
+    // per SM do not (N=1024, 1024 angles, 512 blocks: 1999 / 1775).
+    const long long blocks = (long long)grid.x * grid.y * grid.z, sms = device_sms();
+    if (blocks > 3 * sms && blocks <= 4 * sms) sirt_bp_stack_kernel<4><<<grid, 256, 0, stream>>>(q, it, tol2, active);
+    else sirt_bp_stack_kernel<3><<<grid, 256, 0, stream>>>(q, it, tol2, active);
     return cudaGetLastError();
 }
 
