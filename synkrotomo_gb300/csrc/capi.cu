@@ -277,7 +277,18 @@ int valid_split(int s) { return s == 1 || s == 2 || s == 4 || s == 8; }
 // problem table is uploaded from it (a copy a CUDA graph can capture) instead
 // of from pageable memory.
 // Engine choice by the work per iteration (FP ray-row steps + BP pixel-angle
-// pairs), measured on GB300 with both engines forced on the same inputs:
+// pairs), measured on GB300 on the same inputs.  One problem with deltarho 1:
+// - one slice up to kSmallSingle, and stacks up to kSmallStack: all iterations in
+//   one cooperative launch (sirt_small.cu, at most 360 angles).  us per
+//   iteration, there / two launches per iteration: N=64, 64 angles 8.9 / 12.7;
+//   N=128, 128 angles 12.9 / 17.8; N=256, 360 angles 62 / 76; N=512, 180 angles
+//   (1.1e8) 108 / 156; N=512, 360 angles (2.3e8) 189 / 273; N=768, 180 angles
+//   (2.6e8) 224 / 224; N=1024, 180 angles (4.6e8) 358 / 356.
+// - stacks above it: interleaved slices (sirt_slices.cu); there / one launch:
+//   N=96, 90 angles, 16 slices (3.2e7) 66 / 50; N=256, 180 angles, 2 slices
+//   (5.7e7) 81 / 61; N=256, 60 angles, 8 slices (7.6e7) 76 / 91; N=64, 64 angles,
+//   128 slices (8.1e7) 77 / 111.
+// Otherwise (other spacings, more angles, engine forced, several problems):
 // - up to kSmallWork the phase-split engine with the generic forward phase
 //   (two launches per iteration, no grid barrier) beats the persistent kernel
 //   1.08-1.32x (N=64-256, 1-64 slices);
@@ -286,12 +297,8 @@ int valid_split(int s) { return s == 1 || s == 2 || s == 4 || s == 8; }
 //   N=2048 / 1 slice even); batches of several problems keep the persistent
 //   kernel there.
 constexpr double kSmallWork = 6.0e7;
-// - a stack of at least two slices (deltarho 1) runs on the interleaved-slice
-//   kernels from kSmallStack on, where they pass the generic phases: us per
-//   iteration, generic / interleaved, N=128, 128 angles, 4 slices (2.0e7) 43 /
-//   65; N=64, 64 angles, 32 slices (2.0e7) 48 / 53; N=96, 90 angles, 16 slices
-//   (3.2e7) 70 / 66; N=512, 30 angles, 2 slices (3.8e7) 99 / 67.
-constexpr double kSmallStack = 2.8e7;
+constexpr double kSmallStack = 6.5e7;
+constexpr double kSmallSingle = 2.5e8;
 
 int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double tol, int grid_blocks,
                void *staging = nullptr) {
@@ -340,8 +347,16 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
     const bool slices = fits && in[0].nslices >= 2 && work > kSmallStack && in[0].deltarho == 1.0f &&
                         slices_fit(make_geom(in[0].a, in[0].rhozero, in[0].deltarho, in[0].numrhos, in[0].size,
                                              nullptr));
+    // one small problem (or stack): every iteration in one cooperative launch
+    const int small_grid = grid_blocks == 0 && split && nprob == 1 && !slices &&
+                                   work <= (in[0].nslices >= 2 ? kSmallStack : kSmallSingle) &&
+                                   in[0].deltarho == 1.0f && in[0].a <= kSirtSmallAngles &&
+                                   in[0].iterations < (1 << 20)
+                               ? sirt_small_grid()
+                               : 0;
+    const bool small = small_grid > 0;
     // one large problem: the split engine's forward phase on the projector's own grid
-    const bool stack = slices || (fits && work > kSmallWork);
+    const bool stack = slices || (fits && work > kSmallWork && !small);
     // the work splits fill the warps of the engine that runs the phases
     const long long fp_warps = split ? (long long)fpg * 8 : resident_warps;
     const long long bp_warps = split ? (long long)bpg * 8 : resident_warps;
@@ -386,7 +401,7 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         SYNK_CUDA(sc.get(&R, pr), "cudaMallocAsync(R)");
         SYNK_CUDA(sc.get(&C, n), "cudaMallocAsync(C)");
         // slices: xpad, xTpad and rr hold interleaved slice groups
-        const size_t npx = slices ? slices_floats(np, q.nslices) : np * q.nslices;
+        const size_t npx = slices ? slices_floats(np, q.nslices) : np * q.nslices + (small ? 8 : 0);
         const size_t nrr = slices ? slices_floats(pr, q.nslices) : pr * q.nslices;
         SYNK_CUDA(sc.get(&xpad, npx), "cudaMallocAsync(padded image)");
         SYNK_CUDA(sc.get(&xTpad, npx), "cudaMallocAsync(padded transposed image)");
@@ -418,6 +433,11 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
             if (q.image) SYNK_CUDA(launch_slices_load(q.out, xpad, xTpad, q.size, q.nslices, st), "load kernel");
         } else {
             SYNK_CUDA(launch_pad(q.out, xpad, xTpad, q.size, q.nslices, st), "pad kernel");
+            if (small) {
+                // a clamped gather of the last row reads one entry past the image
+                SYNK_CUDA(cudaMemsetAsync(xpad + np * q.nslices, 0, 8 * sizeof(float), st), "memset");
+                SYNK_CUDA(cudaMemsetAsync(xTpad + np * q.nslices, 0, 8 * sizeof(float), st), "memset");
+            }
         }
         SYNK_CUDA(launch_sumsq(q.projections, pr, q.nslices, b2, st), "norm kernel");
         h.R = R;
@@ -513,7 +533,21 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
     sp.tol2 = tol > 0.0 ? tol * tol : 0.0;
     sp.record_final = want_res ? 1 : 0;
     sp.dynamic = nprob > 1 ? 1 : 0;
-    if (split) {
+    if (small) {
+        SirtSmall ss;
+        ss.q = host[0];
+        sirt_small_splits(host[0].P, host[0].nslices, small_grid, &ss.S, &ss.SB);
+        if (in[0].fp_split) ss.S = in[0].fp_split;
+        if (in[0].bp_split) ss.SB = in[0].bp_split;
+        ss.count = words;
+        ss.extra = ctx->barrier_extra;
+        ss.status = ctx->d_status;
+        ss.timeout_ns = ctx->barrier_timeout_ns;
+        ss.tol2 = sp.tol2;
+        ss.record_final = sp.record_final;
+        ss.want_e2 = sp.tol2 > 0.0 || want_res ? 1 : 0;
+        SYNK_CUDA(launch_sirt_small(ss, small_grid, st), "small SIRT kernel");
+    } else if (split) {
         sp.dynamic = 0;
         int *active = reinterpret_cast<int *>(words + 7);
         // the early exit reads the active count on the host: not inside a graph

@@ -33,11 +33,6 @@
 
 namespace synk {
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 __device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -46,12 +41,6 @@ __device__ __forceinline__ unsigned atom_add_acqrel_u32(unsigned *p, unsigned v)
     asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
     return old;
 }
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 // Grid-wide barrier with a time limit.  Returns false (in every thread of the
 // block) once the barrier or any other block has failed.
 __device__ bool grid_barrier(unsigned *bar, unsigned nblocks, int *status, unsigned long long timeout_ns,

@@ -1,9 +1,20 @@
-// Device functions that the SIRT kernels share (sirt.cu, sirt_slices.cu).
+// Device functions that the SIRT kernels share (sirt.cu, sirt_slices.cu, sirt_small.cu).
 #pragma once
 
 #include "sirt_internal.cuh"
 
 namespace synk {
+
+__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
 
 __device__ __forceinline__ double warp_sum_d(double v) {
 #pragma unroll

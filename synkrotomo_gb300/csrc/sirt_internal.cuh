@@ -56,6 +56,22 @@ struct SirtParams {
     int dynamic;          // hand out items with an atomic counter (uneven batches)
 };
 
+// One small problem in one cooperative launch (sirt_small.cu): deltarho 1, at most kSirtSmallAngles angles.
+constexpr int kSirtSmallAngles = 360;
+struct SirtSmall {
+    SirtProblem q;
+    int S, SB;                // row parts of a ray, angle parts of a pixel
+    unsigned *count;          // barrier arrivals, zero at the launch
+    unsigned extra;           // arrivals every barrier waits for beyond the grid's (fault injection; 0)
+    int *status;              // SYNK_OK or SYNK_ETIMEOUT
+    unsigned long long timeout_ns;
+    double tol2;
+    int record_final, want_e2;
+};
+int sirt_small_grid();        // its blocks (one per SM); 0 if it cannot be resident
+void sirt_small_splits(const ProbGeom &P, int nslices, int grid, int *S, int *SB);
+cudaError_t launch_sirt_small(const SirtSmall &p, int grid, cudaStream_t stream);
+
 cudaError_t launch_sumsq(const float *b, size_t len, int nslices, double *out, cudaStream_t stream);
 cudaError_t launch_sirt_plan(SirtProblem *probs, int nprob, long long *totals, cudaStream_t stream);
 int sirt_persistent_grid(int *blocks_per_sm);
