@@ -5,9 +5,9 @@
 //   warp 0      TMA producer: per K chunk one A box and one B box into a
 //               shared-memory stage (canonical K-major swizzled layout),
 //               completion counted on the stage's "full" mbarrier
-//   warp 1      MMA issuer (one thread): tcgen05.mma kind::f16 per 16-wide K
-//               step, tcgen05.commit frees the stage ("empty" mbarrier), a last
-//               commit signals the accumulator
+//   warp 1      MMA issuer (the warp walks, one elected lane issues): tcgen05.mma
+//               kind::f16 per 16-wide K step, tcgen05.commit frees the stage
+//               ("empty" mbarrier), a last commit signals the accumulator
 //   warps 2-5   epilogue: tcgen05.ld of their 32 TMEM lanes, fused bias / ReLU /
 //               ReLU-mask / atomic accumulation, stores
 // Operand modes (how the producer addresses A and B):
@@ -76,6 +76,24 @@ __device__ __forceinline__ TileInfo tile_info(const GemmParams &p, long long t) 
         ti.nk = (int)(nbk * (ks + 1) / p.ksplit) - ti.kbeg;
     }
     return ti;
+}
+
+// KS K steps of one chunk (one 128- or 64-byte row span): descriptors advance
+// by 32 bytes a step; `acc` false overwrites the accumulator at the first one.
+template <int KS>
+__device__ __forceinline__ void mma_steps(uint32_t dt, uint32_t al, uint32_t bl, uint32_t hi, uint32_t idesc, bool acc) {
+#pragma unroll
+    for (uint32_t kk = 0; kk < (uint32_t)KS; ++kk)
+        mma_bf16(dt, al + 2u * kk, hi, bl + 2u * kk, hi, idesc, kk != 0u || acc ? 1u : 0u);
+}
+// The three taps of one strip: tap kx starts kx rows (128 bytes) into the
+// strip and bTap16 * 16 bytes further into the weights.
+template <int KS>
+__device__ __forceinline__ void mma_taps(uint32_t dt, uint32_t al, uint32_t bl, uint32_t bTap16, uint32_t hi,
+                                         uint32_t idesc, bool acc) {
+#pragma unroll
+    for (uint32_t kx = 0; kx < 3u; ++kx)
+        mma_steps<KS>(dt, al + 8u * kx, bl + kx * bTap16, hi, idesc, kx != 0u || acc);
 }
 
 // Persistent: one CTA per SM walks tiles t = blockIdx.x, += gridDim.x.  The
@@ -202,64 +220,79 @@ __global__ void __launch_bounds__(192, 1) umma_kernel(const __grid_constant__ CU
             if (MODE == MODE_HALO && p.bres) mbar_drain(bfull, 0u, p.limit_ns);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // ---- MMA issuer ----
-            const uint32_t idesc = idesc_bf16(128, p.N);
-            const uint32_t kbytes = (uint32_t)p.kbytes;
-            long long g = 0;
-            int li = 0;
-            bool fail = false;
-            if (MODE == MODE_HALO && p.bres && !mbar_wait(bfull, 0u, p.err, p.limit_ns)) fail = true;
-            for (long long t = blockIdx.x; t < ntiles && !fail; t += gridDim.x, ++li) {
-                const TileInfo ti = tile_info<MODE>(p, t);
-                const int ab = li & 1;
-                const uint32_t dt = tmem + (uint32_t)(ab * p.ncols);
-                if (li >= 2 && !mbar_wait(&tempty[ab], (uint32_t)((li >> 1) - 1) & 1u, p.err, p.limit_ns)) break;
+        // ---- MMA issuer: the whole warp walks and waits, one elected lane issues ----
+        // Issue was what bounded the 3x3 layers: with a `lane == 0` thread that
+        // built both descriptors per step, an MMA took 140-270 cycles at any N
+        // (the tensor pipe needs 16-64 of them).  An elected lane and unrolled steps
+        // on 32-bit descriptor halves: batch 8 at 256 x 256 forward 791 -> 565 us,
+        // training step of 32 images 9.50 -> 7.27 ms.
+        const uint32_t idesc = idesc_bf16(128, p.N);
+        const uint32_t kbytes = (uint32_t)p.kbytes;
+        const uint32_t hi = smem_desc_hi(kbytes);
+        const uint32_t base = smem_u32(smem);
+        uint32_t s = 0, ph = 0;   // stage and its phase parity
+        int li = 0;
+        bool fail = false;
+        if (MODE == MODE_HALO && p.bres) fail = !__all_sync(0xffffffffu, mbar_wait(bfull, 0u, p.err, p.limit_ns));
+        for (long long t = blockIdx.x; t < ntiles && !fail; t += gridDim.x, ++li) {
+            const TileInfo ti = tile_info<MODE>(p, t);
+            const int ab = li & 1;
+            const uint32_t dt = tmem + (uint32_t)(ab * p.ncols);
+            if (li >= 2 && !__all_sync(0xffffffffu, mbar_wait(&tempty[ab], (uint32_t)((li >> 1) - 1) & 1u, p.err,
+                                                              p.limit_ns)))
+                break;
+            tc_fence_after();
+            for (int kc = 0; kc < ti.nk; ++kc) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, p.err, p.limit_ns))) {
+                    fail = true;
+                    break;
+                }
                 tc_fence_after();
-                for (int kc = 0; kc < ti.nk; ++kc, ++g) {
-                    const int s = (int)(g % S);
-                    const uint32_t ph = (uint32_t)(g / S) & 1u;
-                    if (!mbar_wait(&full[s], ph, p.err, p.limit_ns)) {
-                        fail = true;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a0 = smem_u32(smem + (size_t)s * stageBytes);
-                    const uint32_t b0 = a0 + aBytes;
+                const uint32_t a0 = base + s * stageBytes;
+                const uint32_t b0 = a0 + aBytes;
+                if (elect_one()) {
                     if (MODE == MODE_HALO) {
                         // tap kx reads the strip from row kx (pixel w0+kx-1); only the
-                        // chunk's valid channels (32 or 64) are multiplied
+                        // chunk's valid channels (32 or 64) are multiplied; the weights of
+                        // tap (ky, kx): resident block (cc*9 + 3ky + kx) or the stage's box kx
                         const int ky = kc / p.cchunks, cc = kc - ky * p.cchunks;
-                        const uint32_t ksteps = (uint32_t)min(64, p.Cin - 64 * cc) / 16u;
-                        // weights of tap (ky, kx): resident block (cc*9 + 3ky + kx) or the stage's box kx
                         const uint32_t bt0 = p.bres ? smem_u32(bres) + (uint32_t)(cc * 9 + 3 * ky) * bTap : b0;
-                        for (uint32_t kx = 0; kx < 3u; ++kx)
-                            for (uint32_t kk = 0; kk < ksteps; ++kk)
-                                mma_bf16(dt, smem_desc_sw128_at(a0 + kx * 128u + kk * 32u),
-                                         smem_desc(bt0 + kx * bTap + kk * 32u, 128u), idesc,
-                                         (kc | (int)kx | (int)kk) != 0 ? 1u : 0u);
-                    } else if (MODE == MODE_WGRAD) {
-                        // sub-chunk j of the stage: A rows at j*arows, B rows at j*N
-                        const uint32_t nsub = (uint32_t)(p.kw * p.kh);
-                        for (uint32_t j = 0; j < nsub; ++j)
-                            for (uint32_t kk = 0; kk < kbytes / 32u; ++kk)
-                                mma_bf16(dt, smem_desc(a0 + j * (uint32_t)p.arows * kbytes + kk * 32u, kbytes),
-                                         smem_desc(b0 + j * (uint32_t)p.N * kbytes + kk * 32u, kbytes), idesc,
-                                         (kc | (int)j | (int)kk) != 0 ? 1u : 0u);
+                        const uint32_t al = smem_desc_lo(a0), bl = smem_desc_lo(bt0);
+                        if (p.Cin - 64 * cc >= 64)
+                            mma_taps<4>(dt, al, bl, bTap >> 4, hi, idesc, kc != 0);
+                        else
+                            mma_taps<2>(dt, al, bl, bTap >> 4, hi, idesc, kc != 0);
                     } else {
-                        for (uint32_t kk = 0; kk < kbytes / 32u; ++kk) {
-                            mma_bf16(dt, smem_desc(a0 + kk * 32u, kbytes), smem_desc(b0 + kk * 32u, kbytes), idesc,
-                                     (kc | (int)kk) != 0 ? 1u : 0u);
+                        // MODE_WGRAD: sub-chunk j of the stage has its A rows at j*arows, its B rows at j*N
+                        const uint32_t nsub = MODE == MODE_WGRAD ? (uint32_t)(p.kw * p.kh) : 1u;
+                        for (uint32_t j = 0; j < nsub; ++j) {
+                            const uint32_t al = smem_desc_lo(a0 + j * (uint32_t)p.arows * kbytes);
+                            const uint32_t bl = smem_desc_lo(b0 + j * (uint32_t)p.N * kbytes);
+                            if (kbytes == 128u)
+                                mma_steps<4>(dt, al, bl, hi, idesc, (kc | (int)j) != 0);
+                            else
+                                mma_steps<2>(dt, al, bl, hi, idesc, (kc | (int)j) != 0);
                         }
                     }
                     mma_commit(&empty[s]);
+                    if (kc == ti.nk - 1) mma_commit(&tfull[ab]);
                 }
-                if (!fail) mma_commit(&tfull[ab]);
+                __syncwarp();
+                if (++s == (uint32_t)S) {
+                    s = 0;
+                    ph ^= 1u;
+                }
             }
-            // every issued MMA has completed before TMEM is freed
+            // a split-K tile with no chunks: nothing was issued into its buffer
+            if (!fail && ti.nk <= 0 && elect_one()) mma_commit(&tfull[ab]);
+            __syncwarp();
+        }
+        // every issued MMA has completed before TMEM is freed
+        if (elect_one()) {
             mma_commit(drain);
             mbar_drain(drain, 0u, p.limit_ns);
         }
+        __syncwarp();
     } else {
         // ---- epilogue (warps 2..5): TMEM lanes 32*(warp % 4) .. +31 ----
         const int q = warp & 3;
