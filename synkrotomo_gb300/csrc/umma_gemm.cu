@@ -156,24 +156,34 @@ __global__ void __launch_bounds__(192, 1) umma_kernel(const __grid_constant__ CU
     const long long ntiles = p.ntiles;
 
     if (warp == 0) {
-        if (lane == 0) {
-            // ---- TMA producer ----
-            long long g = 0;   // chunks issued by this CTA
-            bool fail = false;
-            if (MODE == MODE_HALO && p.bres) {
-                // all taps' weights once for the CTA's lifetime (one n tile)
-                mbar_arrive_expect_tx(bfull, p.bres);
-                tma_load_3d(bres, &tmB, bfull, 0, 0, 0);
+        // ---- TMA producer: the whole warp walks and waits, one elected lane issues ----
+        uint32_t s = 0, ph = 1;   // stage and the parity of its "empty" phase (fresh barriers pass parity 1)
+        uint32_t used = 0;        // stages filled at least once
+        bool fail = false;
+        if (MODE == MODE_HALO && p.bres && elect_one()) {
+            // all taps' weights once for the CTA's lifetime (one n tile)
+            mbar_arrive_expect_tx(bfull, p.bres);
+            tma_load_3d(bres, &tmB, bfull, 0, 0, 0);
+        }
+        __syncwarp();
+        for (long long t = blockIdx.x; t < ntiles && !fail; t += gridDim.x) {
+            const TileInfo ti = tile_info<MODE>(p, t);
+            int c1 = 0, c2 = 0;   // MODE_HALO: (ky, channel chunk); MODE_CONV: (tap, channel chunk)
+            // MODE_WGRAD: image, row block and column block of the chunk
+            int bb = 0, hb = 0, wb = 0;
+            if (MODE == MODE_WGRAD) {
+                const int per_img = p.nb_h * p.nb_w;
+                bb = ti.kbeg / per_img;
+                const int r = ti.kbeg - bb * per_img;
+                hb = r / p.nb_w;
+                wb = r - hb * p.nb_w;
             }
-            for (long long t = blockIdx.x; t < ntiles && !fail; t += gridDim.x) {
-                const TileInfo ti = tile_info<MODE>(p, t);
-                for (int kc = 0; kc < ti.nk; ++kc) {
-                    const int s = (int)(g % S);
-                    const uint32_t ph = (uint32_t)(g / S) & 1u;
-                    if (g >= S && !mbar_wait(&empty[s], ph ^ 1u, p.err, p.limit_ns)) {
-                        fail = true;
-                        break;
-                    }
+            for (int kc = 0; kc < ti.nk; ++kc) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ph, p.err, p.limit_ns))) {
+                    fail = true;
+                    break;
+                }
+                if (elect_one()) {
                     uint8_t *As = smem + (size_t)s * stageBytes;
                     uint8_t *Bs = As + aBytes;
                     mbar_arrive_expect_tx(&full[s], p.bytesA + p.bytesB);
@@ -186,22 +196,15 @@ __global__ void __launch_bounds__(192, 1) umma_kernel(const __grid_constant__ CU
                         // pixels w0-1 .. w0+128, and the weights of taps (ky, 0..2)
                         // (64-channel boxes; channels >= Cin are out of bounds and read as 0)
                         // B: packed weights [chunk][tap][Cout][64]; the three taps of row ky
-                        // are one box (few large TMA operations keep the copy engine busy)
-                        const int ky = kc / p.cchunks, cc = kc - ky * p.cchunks;
-                        tma_load_4d(As, &tmA, &full[s], cc * 64, ti.w0 - 1, ti.h0 + ky - 1, ti.b);
-                        if (!p.bres) tma_load_3d(Bs, &tmB, &full[s], 0, ti.n0, cc * 9 + 3 * ky);
+                        // are one box
+                        tma_load_4d(As, &tmA, &full[s], c2 * 64, ti.w0 - 1, ti.h0 + c1 - 1, ti.b);
+                        if (!p.bres) tma_load_3d(Bs, &tmB, &full[s], 0, ti.n0, c2 * 9 + 3 * c1);
                     } else if (MODE == MODE_CONV) {
-                        const int tap = kc / p.cchunks, cc = kc - tap * p.cchunks;
-                        const int tky = tap / 3, tkx = tap - tky * 3;
+                        const int tky = c1 / 3, tkx = c1 - tky * 3;
                         const int cw = p.kbytes / 2;   // channels per chunk
-                        tma_load_4d(As, &tmA, &full[s], cc * cw, ti.w0 + tkx - 1, ti.h0 + tky - 1, ti.b);
-                        tma_load_2d(Bs, &tmB, &full[s], tap * p.Cin + cc * cw, ti.n0);
+                        tma_load_4d(As, &tmA, &full[s], c2 * cw, ti.w0 + tkx - 1, ti.h0 + tky - 1, ti.b);
+                        tma_load_2d(Bs, &tmB, &full[s], c1 * p.Cin + c2 * cw, ti.n0);
                     } else {
-                        const int pb = ti.kbeg + kc;
-                        const int per_img = p.nb_h * p.nb_w;
-                        const int bb = pb / per_img;
-                        const int r = pb - bb * per_img;
-                        const int hb = r / p.nb_w, wb = r - (r / p.nb_w) * p.nb_w;
                         // blocked operands [image][row][pixel chunk][channel][pixel]: a box is
                         // one contiguous block; the tap's row shift is the H coordinate (zero
                         // outside the image) and its column shift the pre-shifted copy kx
@@ -210,15 +213,35 @@ __global__ void __launch_bounds__(192, 1) umma_kernel(const __grid_constant__ CU
                         tma_load_5d(Bs, &tmB, &full[s], 0, ti.n0, wb * p.kw, hb * p.kh + ti.ky - 1,
                                     ti.kx * p.Bn + bb);
                     }
-                    ++g;
+                }
+                __syncwarp();
+                if (MODE == MODE_HALO || MODE == MODE_CONV) {
+                    if (++c2 == p.cchunks) {
+                        c2 = 0;
+                        ++c1;
+                    }
+                } else if (MODE == MODE_WGRAD) {
+                    if (++wb == p.nb_w) {
+                        wb = 0;
+                        if (++hb == p.nb_h) {
+                            hb = 0;
+                            ++bb;
+                        }
+                    }
+                }
+                if (used < (uint32_t)S) ++used;
+                if (++s == (uint32_t)S) {
+                    s = 0;
+                    ph ^= 1u;
                 }
             }
-            // no copy may still be landing when the CTA exits: wait (bounded) for
-            // the last use of every stage (immediate on the normal path)
-            const long long first = g > S ? g - S : 0;
-            for (long long c = first; c < g; ++c) mbar_drain(&full[c % S], (uint32_t)(c / S) & 1u, p.limit_ns);
-            if (MODE == MODE_HALO && p.bres) mbar_drain(bfull, 0u, p.limit_ns);
         }
+        // no copy may still be landing when the CTA exits: wait (bounded) for
+        // the last use of every stage (immediate on the normal path); the
+        // stages below s were last filled in the current round, the others in the one before
+        for (uint32_t c = 0; c < used; ++c) mbar_drain(&full[c], c < s ? ph ^ 1u : ph, p.limit_ns);
+        if (MODE == MODE_HALO && p.bres) mbar_drain(bfull, 0u, p.limit_ns);
+        __syncwarp();
     } else if (warp == 1) {
         // ---- MMA issuer: the whole warp walks and waits, one elected lane issues ----
         // Issue was what bounded the 3x3 layers: with a `lane == 0` thread that
