@@ -116,6 +116,24 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, u
         "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
         : "memory");
 }
+// Shared -> global, completion by bulk group of the issuing thread.
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, const void *src, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(map),
+        "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+        : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// All but the newest KEEP groups of this thread have left shared memory.
+template <int KEEP>
+__device__ __forceinline__ void bulk_wait_read() {
+    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(KEEP) : "memory");
+}
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+// Orders this thread's shared-memory writes before later copies of them.
+__device__ __forceinline__ void fence_async_shared() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
@@ -183,6 +201,30 @@ __device__ __forceinline__ bool elect_one() {
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok));
     return ok != 0;
+}
+// KS K steps of one chunk (one row span): descriptors advance by 32 bytes a
+// step; `acc` false overwrites the accumulator at the first one.
+template <int KS>
+__device__ __forceinline__ void mma_steps(uint32_t dt, uint32_t al, uint32_t bl, uint32_t hi, uint32_t idesc, bool acc) {
+#pragma unroll
+    for (uint32_t kk = 0; kk < (uint32_t)KS; ++kk)
+        mma_bf16(dt, al + 2u * kk, hi, bl + 2u * kk, hi, idesc, kk != 0u || acc ? 1u : 0u);
+}
+// The three taps of one strip with rows of ROW bytes: tap kx starts kx rows
+// into the strip and kx * tap16 * 16 bytes further into the weights; 4 or 2 K steps.
+template <int ROW>
+__device__ __forceinline__ void mma_taps(bool four, uint32_t dt, uint32_t al, uint32_t bl, uint32_t tap16, uint32_t hi,
+                                         uint32_t idesc, bool acc) {
+    constexpr uint32_t kRow16 = ROW / 16;
+    if (ROW == 128 && four) {
+#pragma unroll
+        for (uint32_t kx = 0; kx < 3u; ++kx)
+            mma_steps<4>(dt, al + kRow16 * kx, bl + kx * tap16, hi, idesc, kx != 0u || acc);
+    } else {
+#pragma unroll
+        for (uint32_t kx = 0; kx < 3u; ++kx)
+            mma_steps<2>(dt, al + kRow16 * kx, bl + kx * tap16, hi, idesc, kx != 0u || acc);
+    }
 }
 // Arrives on `bar` once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {

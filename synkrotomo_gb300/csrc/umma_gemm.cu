@@ -78,24 +78,6 @@ __device__ __forceinline__ TileInfo tile_info(const GemmParams &p, long long t) 
     return ti;
 }
 
-// KS K steps of one chunk (one 128- or 64-byte row span): descriptors advance
-// by 32 bytes a step; `acc` false overwrites the accumulator at the first one.
-template <int KS>
-__device__ __forceinline__ void mma_steps(uint32_t dt, uint32_t al, uint32_t bl, uint32_t hi, uint32_t idesc, bool acc) {
-#pragma unroll
-    for (uint32_t kk = 0; kk < (uint32_t)KS; ++kk)
-        mma_bf16(dt, al + 2u * kk, hi, bl + 2u * kk, hi, idesc, kk != 0u || acc ? 1u : 0u);
-}
-// The three taps of one strip: tap kx starts kx rows (128 bytes) into the
-// strip and bTap16 * 16 bytes further into the weights.
-template <int KS>
-__device__ __forceinline__ void mma_taps(uint32_t dt, uint32_t al, uint32_t bl, uint32_t bTap16, uint32_t hi,
-                                         uint32_t idesc, bool acc) {
-#pragma unroll
-    for (uint32_t kx = 0; kx < 3u; ++kx)
-        mma_steps<KS>(dt, al + 8u * kx, bl + kx * bTap16, hi, idesc, kx != 0u || acc);
-}
-
 // Persistent: one CTA per SM walks tiles t = blockIdx.x, += gridDim.x.  The
 // shared-memory stage ring runs continuously across tiles, and the FP32
 // accumulator is double-buffered in TMEM (2 x ncols columns): the MMA warp
@@ -163,7 +145,8 @@ __global__ void __launch_bounds__(192, 1) umma_kernel(const __grid_constant__ CU
         if (MODE == MODE_HALO && p.bres && elect_one()) {
             // all taps' weights once for the CTA's lifetime (one n tile)
             mbar_arrive_expect_tx(bfull, p.bres);
-            tma_load_3d(bres, &tmB, bfull, 0, 0, 0);
+            for (int cc = 0; cc < p.cchunks; ++cc)
+                tma_load_3d(bres + (size_t)cc * 9 * bTap, &tmB, bfull, cc * 64, 0, 0);
         }
         __syncwarp();
         for (long long t = blockIdx.x; t < ntiles && !fail; t += gridDim.x) {
@@ -195,10 +178,9 @@ __global__ void __launch_bounds__(192, 1) umma_kernel(const __grid_constant__ CU
                         // chunk = (ky, channel chunk cc): the strip of row h0+ky-1,
                         // pixels w0-1 .. w0+128, and the weights of taps (ky, 0..2)
                         // (64-channel boxes; channels >= Cin are out of bounds and read as 0)
-                        // B: packed weights [chunk][tap][Cout][64]; the three taps of row ky
-                        // are one box
+                        // B: the three taps of row ky are one box
                         tma_load_4d(As, &tmA, &full[s], c2 * 64, ti.w0 - 1, ti.h0 + c1 - 1, ti.b);
-                        if (!p.bres) tma_load_3d(Bs, &tmB, &full[s], 0, ti.n0, c2 * 9 + 3 * c1);
+                        if (!p.bres) tma_load_3d(Bs, &tmB, &full[s], c2 * 64, ti.n0, 3 * c1);
                     } else if (MODE == MODE_CONV) {
                         const int tky = c1 / 3, tkx = c1 - tky * 3;
                         const int cw = p.kbytes / 2;   // channels per chunk
@@ -281,10 +263,7 @@ __global__ void __launch_bounds__(192, 1) umma_kernel(const __grid_constant__ CU
                         const int ky = kc / p.cchunks, cc = kc - ky * p.cchunks;
                         const uint32_t bt0 = p.bres ? smem_u32(bres) + (uint32_t)(cc * 9 + 3 * ky) * bTap : b0;
                         const uint32_t al = smem_desc_lo(a0), bl = smem_desc_lo(bt0);
-                        if (p.Cin - 64 * cc >= 64)
-                            mma_taps<4>(dt, al, bl, bTap >> 4, hi, idesc, kc != 0);
-                        else
-                            mma_taps<2>(dt, al, bl, bTap >> 4, hi, idesc, kc != 0);
+                        mma_taps<128>(p.Cin - 64 * cc >= 64, dt, al, bl, bTap >> 4, hi, idesc, kc != 0);
                     } else {
                         // MODE_WGRAD: sub-chunk j of the stage has its A rows at j*arows, its B rows at j*N
                         const uint32_t nsub = MODE == MODE_WGRAD ? (uint32_t)(p.kw * p.kh) : 1u;
@@ -523,24 +502,8 @@ cudaError_t gemm_bf16(const uint16_t *A, const uint16_t *B, float *C, int M, int
     return launch<MODE_GEMM, EPI_F32>(ta, tb, p, dim3(M / 128, 1, 1), st);
 }
 
-// wp[(cc*9 + tap)*Cout + o][j] = w[o][tap*Cin + 64*cc + j] (0 past Cin): the
-// weights of the row-strip form, 64-channel chunks, taps and output channels
-// as rows of 128 bytes.
-__global__ void pack_weights_kernel(const uint16_t *__restrict__ w, uint16_t *__restrict__ wp, int Cin, int Cout,
-                                    int cchunks) {
-    const long long n = (long long)cchunks * 9 * Cout * 64;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(i & 63);
-        const long long r = i >> 6;
-        const int o = (int)(r % Cout);
-        const int t = (int)(r / Cout);          // cc*9 + tap
-        const int cc = t / 9, tap = t - cc * 9;
-        const int c = 64 * cc + j;
-        wp[i] = c < Cin ? w[(long long)o * 9 * Cin + tap * Cin + c] : (uint16_t)0;
-    }
-}
-
-// Image rows of 128k pixels: a tile is 128 pixels of one row, and per input
+// Layers of long rows whose weights do not fit in shared memory beside the
+// strips (192 -> 64 and wider; the others take conv_rows): a tile is 128 pixels of one row, and per input
 // row ky and 64-channel chunk ONE strip of 130 pixels (halo of one on each
 // side) is loaded, with the three taps' weights as one more box; the taps kx
 // are views of the strip shifted by kx rows.  Compared with a box per tap
@@ -582,34 +545,40 @@ static cudaError_t conv3x3_halo(const ConvArgs &c, int epi, int ntile, int *err,
     p.moff = c.moff;
     p.err = err;
     p.limit_ns = limit_ns;
-    // packed weights in stream-ordered scratch
-    const long long npk = (long long)p.cchunks * 9 * c.Cout * 64;
-    uint16_t *wp = nullptr;
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&wp), (size_t)npk * 2, st);
-    if (e != cudaSuccess) return e;
-    pack_weights_kernel<<<(unsigned)((npk + 255) / 256 < 1024 ? (npk + 255) / 256 : 1024), 256, 0, st>>>(
-        c.w, wp, c.Cin, c.Cout, p.cchunks);
-    if ((e = cudaGetLastError()) != cudaSuccess) {
-        cudaFreeAsync(wp, st);
-        return e;
-    }
     CUtensorMap ta, tb;
     const uint64_t da[4] = {(uint64_t)c.Cin, (uint64_t)c.W, (uint64_t)c.H, (uint64_t)c.B};
     const uint64_t sa[3] = {(uint64_t)c.ldx * 2, (uint64_t)c.ldx * 2 * c.W, (uint64_t)c.ldx * 2 * c.W * c.H};
     const uint32_t ba[4] = {64, 130, 1, 1};
-    const uint64_t db[3] = {64, (uint64_t)c.Cout, (uint64_t)p.cchunks * 9};
-    const uint64_t sb[2] = {128, (uint64_t)c.Cout * 128};
-    const uint32_t bbx[3] = {64, (uint32_t)ntile, resident ? (uint32_t)(p.cchunks * 9) : 3u};
+    // w[o][tap*Cin + i] as (i, o, tap): a box of one channel chunk lands as [tap][o][i]
+    const uint64_t db[3] = {(uint64_t)c.Cin, (uint64_t)c.Cout, 9};
+    const uint64_t sb[2] = {(uint64_t)c.Cin * 18, (uint64_t)c.Cin * 2};
+    const uint32_t bbx[3] = {64, (uint32_t)ntile, resident ? 9u : 3u};
     const dim3 grid((unsigned)((long long)c.B * c.H * c.W / 128), (unsigned)(c.Cout / ntile), 1);
-    if ((e = tensor_map(&ta, c.x + c.xoff, 4, da, sa, ba, 128)) == cudaSuccess &&
-        (e = tensor_map(&tb, wp, 3, db, sb, bbx, 128)) == cudaSuccess) {
-        switch (epi) {
-            case EPI_BIAS_RELU: e = launch<MODE_HALO, EPI_BIAS_RELU>(ta, tb, p, grid, st); break;
-            case EPI_BIAS: e = launch<MODE_HALO, EPI_BIAS>(ta, tb, p, grid, st); break;
-            case EPI_MASK: e = launch<MODE_HALO, EPI_MASK>(ta, tb, p, grid, st); break;
-            default: e = cudaErrorInvalidValue;
-        }
+    cudaError_t e;
+    if ((e = tensor_map(&ta, c.x + c.xoff, 4, da, sa, ba, 128)) != cudaSuccess) return e;
+    if ((e = tensor_map(&tb, c.w, 3, db, sb, bbx, 128)) != cudaSuccess) return e;
+    switch (epi) {
+        case EPI_BIAS_RELU: return launch<MODE_HALO, EPI_BIAS_RELU>(ta, tb, p, grid, st);
+        case EPI_BIAS: return launch<MODE_HALO, EPI_BIAS>(ta, tb, p, grid, st);
+        case EPI_MASK: return launch<MODE_HALO, EPI_MASK>(ta, tb, p, grid, st);
+        default: return cudaErrorInvalidValue;
     }
+}
+
+// The same with the weights at an address that the copies accept.
+static cudaError_t conv3x3_wide(const ConvArgs &c, int epi, int ntile, int *err, unsigned long long limit_ns,
+                                cudaStream_t st) {
+    if ((reinterpret_cast<uintptr_t>(c.w) & 15u) == 0)
+        return conv_rows_fits(c, epi) ? conv_rows(c, epi, err, limit_ns, st)
+                                      : conv3x3_halo(c, epi, ntile, err, limit_ns, st);
+    const size_t bytes = (size_t)c.Cout * 9 * c.Cin * 2;
+    ConvArgs a = c;
+    uint16_t *wp = nullptr;
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&wp), bytes, st);
+    if (e != cudaSuccess) return e;
+    a.w = wp;
+    e = cudaMemcpyAsync(wp, c.w, bytes, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess) e = conv3x3_wide(a, epi, ntile, err, limit_ns, st);
     const cudaError_t e2 = cudaFreeAsync(wp, st);
     return e != cudaSuccess ? e : e2;
 }
@@ -623,7 +592,7 @@ cudaError_t conv3x3(const ConvArgs &c, int epi, int *err, unsigned long long lim
     if (ntile == 0) return cudaErrorInvalidValue;
     // the row-strip form when a tile is one image row and two stages fit
     if (c.W % 128 == 0 && kb_round(130u * 128u) + kb_round(3u * (size_t)ntile * 128u) <= 100u * 1024u)
-        return conv3x3_halo(c, epi, ntile, err, limit_ns, st);
+        return conv3x3_wide(c, epi, ntile, err, limit_ns, st);
     const int bw = c.W >= 128 ? 128 : c.W;
     const int bh = 128 / bw;
     if (128 % bw || c.W % bw || c.H % bh) return cudaErrorInvalidValue;

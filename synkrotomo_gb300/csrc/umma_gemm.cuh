@@ -1,6 +1,7 @@
 // tcgen05 GEMM engine of the U-Net (umma_gemm.cu).
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -59,6 +60,13 @@ struct WgradArgs {
 cudaError_t gemm_bf16(const uint16_t *A, const uint16_t *B, float *C, int M, int N, int K, int *err,
                       unsigned long long limit_ns, cudaStream_t st);
 cudaError_t conv3x3(const ConvArgs &c, int epi, int *err, unsigned long long limit_ns, cudaStream_t st);
+// conv_rows.cu: the form that reads every strip of a long image row once; `fits`
+// says whether its shared memory holds the layer (conv3x3 chooses).
+bool conv_rows_fits(const ConvArgs &c, int epi);
+cudaError_t conv_rows(const ConvArgs &c, int epi, int *err, unsigned long long limit_ns, cudaStream_t st);
+// Tensor map of BF16 rows of row_bytes (64 or 128, swizzled by as much).
+cudaError_t tensor_map(CUtensorMap *m, const void *ptr, int rank, const uint64_t *dims, const uint64_t *strides,
+                       const uint32_t *box, int row_bytes);
 cudaError_t conv3x3_wgrad(const WgradArgs &w, int *err, unsigned long long limit_ns, cudaStream_t st);
 
 }  // namespace unet
