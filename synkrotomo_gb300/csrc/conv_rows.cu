@@ -14,18 +14,23 @@
 //
 //   warp 0      TMA producer of strips        full[s] / empty[s]
 //   warp 1      MMA issuer                    tfull[j] / tempty[j]
-//   warps 2-5   epilogue; results leave by TMA from a shared tile, and in
-//               backward-data the tile first holds the mask (the layer input),
-//               loaded by TMA two rows ahead and overwritten in place: iofull[j]
+//   warps 2-9   two epilogue groups of four warps that take turns at the rows;
+//               results leave by TMA from a shared tile, and in backward-data
+//               the tile first holds the mask (the layer input), loaded by TMA
+//               ahead of time and overwritten in place: iofull[j].  One group's
+//               chain of waits (accumulator, barrier, TMEM, shared memory, copy)
+//               is longer than a row takes to multiply
 //
 // What bounds it: HBM for the narrow layers (the 32-channel ones move 128 to
 // 450 bytes per pixel), the MMA rate for the others: M=128, N<=128 costs 32 + N/4
 // cycles per 16-wide K step, bound by reading the operands from shared memory.
 // Against the tile-by-tile form (a strip per tile and tap row, each strip read
 // three times; epilogue stores and mask loads from registers), 8 / 32 images:
-// 32 -> 32 at 256 x 256 42 -> 31 / 154 -> 109 us, 96 -> 32 82 -> 54 / 311 -> 193,
+// 32 -> 32 at 256 x 256 42 -> 26 / 154 -> 84 us, 96 -> 32 82 -> 54 / 311 -> 192,
 // 64 -> 64 at 128 x 128 19 -> 16 / 57 -> 41; backward-data of 32 images 32 -> 96
-// 367 -> 194, 32 -> 32 172 -> 138, 64 -> 192 at 128 x 128 190 -> 124.
+// 367 -> 169, 32 -> 32 172 -> 104, 64 -> 192 at 128 x 128 190 -> 109 (with one
+// epilogue group 109, 194, 138 and 124 for the 32-image 32 -> 32, 32 -> 96,
+// 32 -> 32 backward and 64 -> 192).
 #include "synk_internal.cuh"
 #include "umma.cuh"
 #include "umma_gemm.cuh"
@@ -34,6 +39,8 @@ namespace synk {
 namespace unet {
 
 using namespace umma;
+
+constexpr uint32_t kTiles = 2;   // shared tiles of an epilogue group
 
 struct RowsParams {
     int N, gy, cchunks, H, tiles_w, last_steps;
@@ -91,19 +98,21 @@ struct RowCursor {
     }
 };
 
-__device__ __forceinline__ bool epi_and(bool v) {
+__device__ __forceinline__ bool epi_and(int id, bool v) {
     uint32_t r;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.u32 p, %1, 0;\n\t"
-        "barrier.cta.red.and.pred q, 1, 128, p;\n\t"
+        "barrier.cta.red.and.pred q, %2, 128, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(r)
-        : "r"(v ? 1u : 0u)
+        : "r"(v ? 1u : 0u), "r"(id)
         : "memory");
     return r != 0;
 }
-__device__ __forceinline__ void epi_sync() { asm volatile("barrier.cta.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void epi_sync(int id) {
+    asm volatile("barrier.cta.sync %0, 128;" ::"r"(id) : "memory");
+}
 
 __device__ __forceinline__ uint32_t bf2(float lo, float hi) {
     uint32_t r;
@@ -114,7 +123,7 @@ __device__ __forceinline__ uint32_t bf2(float lo, float hi) {
 // EPI: EPI_BIAS_RELU, EPI_BIAS or EPI_MASK.  CW: channels per strip (64, or 32
 // for 32-channel inputs: 64-byte rows, half the shared memory and copy work).
 template <int EPI, int CW>
-__global__ void __launch_bounds__(192, 1) conv_rows_kernel(const __grid_constant__ CUtensorMap tmX,
+__global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant__ CUtensorMap tmX,
                                                            const __grid_constant__ CUtensorMap tmW,
                                                            const __grid_constant__ CUtensorMap tmY,
                                                            const __grid_constant__ CUtensorMap tmM,
@@ -276,32 +285,39 @@ __global__ void __launch_bounds__(192, 1) conv_rows_kernel(const __grid_constant
         const uint32_t nb1 = (uint32_t)p.nb - 1u;
         const int nbl = 31 - __clz(p.nb);
         const uint32_t rsw = (uint32_t)((row >> 1) & 3);
-        const bool mover = warp == 2 && elect_one();   // issues the tile's copies
-        RowCursor cur(p, run), ahead(p, run);
+        const int grp = (warp - 2) >> 2, bar = 1 + grp;          // the group takes rows grp, grp + 2, ...
+        const bool mover = ((warp - 2) & 3) == 0 && elect_one();   // issues the group's copies
+        uint8_t *gio = io + (size_t)grp * kTiles * p.io_bytes;
+        uint64_t *gfull = iofull + grp * kTiles;
+        RowCursor cur(p, run);
+        if (grp) cur.next(p);
+        RowCursor ahead = cur;
         uint32_t loads = 0;                            // mask tiles requested (mover only)
         auto load_mask = [&]() {
-            const uint32_t j = loads % (uint32_t)p.nio;
-            mbar_arrive_expect_tx(&iofull[j], p.io_bytes);
+            const uint32_t j = loads % kTiles;
+            mbar_arrive_expect_tx(&gfull[j], p.io_bytes);
             for (int c = 0; c < p.N / 32; ++c)
-                tma_load_4d(io + (size_t)j * p.io_bytes + (size_t)c * 8192u, &tmM, &iofull[j], run.n0 + 32 * c,
+                tma_load_4d(gio + (size_t)j * p.io_bytes + (size_t)c * 8192u, &tmM, &gfull[j], run.n0 + 32 * c,
                             ahead.wt * 128, ahead.h, ahead.b);
             ++loads;
             ahead.next(p);
+            ahead.next(p);
         };
         if (EPI == EPI_MASK && mover)
-            for (int k = 0; k + 1 < p.nio && ahead.left > 0; ++k) load_mask();
-        uint32_t li = 0, j = 0, jph = 0;               // row, its shared tile and that tile's phase
-        for (; cur.left > 0; cur.next(p), ++li) {
+            for (uint32_t k = 0; k + 1 < kTiles && ahead.left > 0; ++k) load_mask();
+        uint32_t li = (uint32_t)grp, j = 0, jph = 0;   // row, its shared tile and that tile's phase
+        for (; cur.left > 0; cur.next(p), cur.next(p), li += 2) {
             bool ok = mbar_wait(&tfull[li & nb1], (li >> nbl) & 1u, p.err, p.limit_ns);
             if (EPI == EPI_MASK) {
-                ok = ok && mbar_wait(&iofull[j], jph, p.err, p.limit_ns);
+                ok = ok && mbar_wait(&gfull[j], jph, p.err, p.limit_ns);
             } else if (mover) {
-                bulk_wait_read<1>();                   // the store that last read this tile (nio = 2) is done
+                bulk_wait_read<kTiles - 1>();          // the store that last read this tile is done
             }
-            // one decision for the four warps
-            if (!epi_and(ok && *(volatile int *)p.err == 0)) break;
+            // one decision for the four warps (an accumulator is only ever signalled whole:
+            // the error word needs no look here, a trip to L2 per row)
+            if (!epi_and(bar, ok)) break;
             tc_fence_after();
-            uint8_t *tile = io + (size_t)j * p.io_bytes;
+            uint8_t *tile = gio + (size_t)j * p.io_bytes;
             const uint32_t tbase = tmem + (li & nb1) * (uint32_t)p.N + ((uint32_t)(q4 * 32) << 16);
             for (int c0 = 0; c0 < p.N; c0 += 32) {
                 float v[32];
@@ -344,7 +360,7 @@ __global__ void __launch_bounds__(192, 1) conv_rows_kernel(const __grid_constant
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty[li & nb1]);
             fence_async_shared();
-            epi_sync();
+            epi_sync(bar);
             if (mover) {
                 for (int c = 0; c < p.N / 32; ++c)
                     tma_store_4d(&tmY, tile + (size_t)c * 8192u, run.n0 + 32 * c, cur.wt * 128, cur.h, cur.b);
@@ -354,7 +370,7 @@ __global__ void __launch_bounds__(192, 1) conv_rows_kernel(const __grid_constant
                     load_mask();
                 }
             }
-            if (++j == (uint32_t)p.nio) {
+            if (++j == kTiles) {
                 j = 0;
                 jph ^= 1u;
             }
@@ -362,8 +378,8 @@ __global__ void __launch_bounds__(192, 1) conv_rows_kernel(const __grid_constant
         if (mover) {
             bulk_wait_all();
             if (EPI == EPI_MASK)   // no copy may still be landing (only after a failure is one in flight)
-                for (uint32_t k = loads > (uint32_t)p.nio ? loads - (uint32_t)p.nio : 0u; k < loads; ++k)
-                    mbar_drain(&iofull[k % (uint32_t)p.nio], (k / (uint32_t)p.nio) & 1u, p.limit_ns);
+                for (uint32_t k = loads > kTiles ? loads - kTiles : 0u; k < loads; ++k)
+                    mbar_drain(&gfull[k % kTiles], (k / kTiles) & 1u, p.limit_ns);
         }
         __syncwarp();
     }
@@ -386,7 +402,7 @@ static bool rows_plan(const ConvArgs &c, int epi, RowsParams &p, size_t *smem) {
     p.last_steps = (c.Cin - cw * (p.cchunks - 1)) / 16;
     p.stage_bytes = kb1(130u * 2 * cw);
     p.strip_tx = 130u * 2 * cw;
-    p.nio = epi == EPI_MASK ? 3 : 2;   // masks are requested two rows ahead
+    p.nio = 2 * (int)kTiles;
     // the widest n tile of at most 128 columns (four accumulators open at a time in 512)
     // that divides Cout and leaves room; below 64 the MMAs cost more than the copies save
     for (int n = c.Cout <= 128 ? c.Cout : 128; n >= (c.Cout < 64 ? 32 : 64); n -= 32) {
@@ -396,7 +412,7 @@ static bool rows_plan(const ConvArgs &c, int epi, RowsParams &p, size_t *smem) {
         p.tap_bytes = (uint32_t)(n * 2 * cw);
         p.w_bytes = p.w_tx = p.cchunks * 9u * p.tap_bytes;
         p.io_bytes = (uint32_t)n * 256u;
-        const size_t fixed = 1024 + p.w_bytes + (size_t)p.nio * p.io_bytes + 8 * (2 * 8 + 2 * 8 + 4) + 16 + 4 * (size_t)n;
+        const size_t fixed = 1024 + p.w_bytes + (size_t)p.nio * p.io_bytes + 8 * (2 * 8 + 2 * 8 + 2 * kTiles + 2) + 16 + 4 * (size_t)n;
         const size_t room = 227u * 1024u;
         if (fixed + 3 * (size_t)p.stage_bytes > room) continue;
         const size_t s = (room - fixed) / p.stage_bytes;
@@ -418,7 +434,7 @@ static cudaError_t rows_launch(const CUtensorMap &x, const CUtensorMap &w, const
     if (e != cudaSuccess) return e;
     const long long most = p.rows * p.gy;
     const int sms = device_sms();
-    conv_rows_kernel<EPI, CW><<<(unsigned)(most < sms ? most : sms), 192, smem, st>>>(x, w, y, m, p);
+    conv_rows_kernel<EPI, CW><<<(unsigned)(most < sms ? most : sms), 320, smem, st>>>(x, w, y, m, p);
     return cudaGetLastError();
 }
 

@@ -305,8 +305,9 @@ __global__ void __launch_bounds__(192, 1) umma_kernel(const __grid_constant__ CU
             const int ab = li & 1;
             const bool ok = mbar_wait(&tfull[ab], (uint32_t)(li >> 1) & 1u, p.err, p.limit_ns);
             tc_fence_after();
-            // tcgen05.ld is warp-collective: decide once per warp
-            const bool good = __all_sync(0xffffffffu, ok && *(volatile int *)p.err == 0);
+            // tcgen05.ld is warp-collective: decide once per warp (an accumulator is only
+            // ever signalled whole: the error word needs no look here, a trip to L2 per tile)
+            const bool good = __all_sync(0xffffffffu, ok);
             if (!good) break;
             // a split-K tile with no chunks contributes nothing (its buffer was not written)
             const int ncol = ti.nk > 0 ? p.N : 0;
