@@ -6,7 +6,8 @@
 // one input row (130 pixels, one halo pixel each side, 64 or 32 channels) feeds
 // the three output rows it touches, whose accumulators are open in TMEM at the
 // same time (a ring of nb buffers of N columns): input row r adds tap row ky=2
-// to output row r-1 (which is then complete), ky=1 to r and ky=0 to r+1.  Each
+// to output row r-1 (which is then complete), ky=1 to r and ky=0 to r+1.  The
+// three are one MMA of 3N columns where the ring does not end between them.  Each
 // output element still adds its products in the order ky, channel chunk, kx,
 // channel, so the results equal those of the tile-by-tile form bit for bit.  The
 // weights of all nine taps stay in shared memory for the CTA's lifetime, read
@@ -22,15 +23,17 @@
 //               is longer than a row takes to multiply
 //
 // What bounds it: HBM for the narrow layers (the 32-channel ones move 128 to
-// 450 bytes per pixel), the MMA rate for the others: M=128, N<=128 costs 32 + N/4
-// cycles per 16-wide K step, bound by reading the operands from shared memory.
+// 450 bytes per pixel; 32 -> 32 reaches 0.55 of it), and shared memory, where the
+// MMAs read their operands (M=128: 32 cycles for A plus N/4 for B per 16-wide K
+// step, and the pipe's N/2 from N=128 on), which is why A is read once for the
+// three tap rows.
 // Against the tile-by-tile form (a strip per tile and tap row, each strip read
 // three times; epilogue stores and mask loads from registers), 8 / 32 images:
-// 32 -> 32 at 256 x 256 42 -> 26 / 154 -> 84 us, 96 -> 32 82 -> 54 / 311 -> 192,
-// 64 -> 64 at 128 x 128 19 -> 16 / 57 -> 41; backward-data of 32 images 32 -> 96
-// 367 -> 169, 32 -> 32 172 -> 104, 64 -> 192 at 128 x 128 190 -> 109 (with one
-// epilogue group 109, 194, 138 and 124 for the 32-image 32 -> 32, 32 -> 96,
-// 32 -> 32 backward and 64 -> 192).
+// 32 -> 32 at 256 x 256 42 -> 24 / 154 -> 74 us, 96 -> 32 82 -> 42 / 311 -> 139,
+// 64 -> 64 at 128 x 128 19 -> 15 / 57 -> 36; backward-data of 32 images 32 -> 96
+// 367 -> 167, 32 -> 32 172 -> 100, 64 -> 192 at 128 x 128 190 -> 106.  Of that,
+// one MMA for the three tap rows: 32 -> 32 84 -> 74, 96 -> 32 192 -> 139; two
+// epilogue groups instead of one: 32 -> 32 109 -> 84.
 #include "synk_internal.cuh"
 #include "umma.cuh"
 #include "umma_gemm.cuh"
@@ -44,9 +47,9 @@ constexpr uint32_t kTiles = 2;   // shared tiles of an epilogue group
 
 struct RowsParams {
     int N, gy, cchunks, H, tiles_w, last_steps;
-    int stages, nb, nio;
+    int stages, nb, nio, at_once;
     long long rows;                              // B * tiles_w * H output rows of 128 pixels
-    uint32_t stage_bytes, strip_tx, w_tx, w_bytes, tap_bytes, io_bytes, tmem_cols;
+    uint32_t stage_bytes, strip_tx, w_tx, w_bytes, tap_bytes, io_bytes;
     const float *bias;
     int *err;
     unsigned long long limit_ns;
@@ -120,6 +123,32 @@ __device__ __forceinline__ uint32_t bf2(float lo, float hi) {
     return r;
 }
 
+// One strip (rows of ROW bytes) times the tap rows of c adjacent accumulators of N
+// columns from dt on: per kx and K step one MMA of c*N columns, so that the
+// strip is read from shared memory once for all of them.  `fresh`: the last
+// accumulator is new and its first product overwrites what it held.
+template <int ROW>
+__device__ __forceinline__ void mma_rows(bool four, uint32_t dt, uint32_t N, uint32_t al, uint32_t bl, uint32_t tap16,
+                                         uint32_t hi, uint32_t c, bool fresh) {
+    const uint32_t id1 = idesc_bf16(128, 0) | ((N >> 3) << 17), idc = idesc_bf16(128, 0) | ((c * N >> 3) << 17);
+    if (fresh) {
+        if (c > 1) mma_bf16(dt, al, hi, bl, hi, idc - ((N >> 3) << 17), 1u);
+        mma_bf16(dt + (c - 1u) * N, al, hi, bl + (c - 1u) * tap16, hi, id1, 0u);
+    } else {
+        mma_bf16(dt, al, hi, bl, hi, idc, 1u);
+    }
+    if (ROW == 128 && four) {
+#pragma unroll
+        for (uint32_t k = 1; k < 12u; ++k)
+            mma_bf16(dt, al + 8u * (k >> 2) + 2u * (k & 3u), hi, bl + 3u * (k >> 2) * tap16 + 2u * (k & 3u), hi, idc, 1u);
+    } else {
+#pragma unroll
+        for (uint32_t k = 1; k < 6u; ++k)
+            mma_bf16(dt, al + (ROW / 16u) * (k >> 1) + 2u * (k & 1u), hi, bl + 3u * (k >> 1) * tap16 + 2u * (k & 1u), hi,
+                     idc, 1u);
+    }
+}
+
 // EPI: EPI_BIAS_RELU, EPI_BIAS or EPI_MASK.  CW: channels per strip (64, or 32
 // for 32-channel inputs: 64-byte rows, half the shared memory and copy work).
 template <int EPI, int CW>
@@ -147,7 +176,7 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const RowRun run(p);
     if (warp == 0) {
-        tmem_alloc(tmem_slot, p.tmem_cols);
+        tmem_alloc(tmem_slot, 512u);
         tmem_relinquish();
     }
     if (warp == 1 && lane == 0) {
@@ -181,8 +210,12 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
         // ---- producer ----
         if (elect_one()) {
             mbar_arrive_expect_tx(wfull, p.w_tx);
+            // [chunk][kx][ky = 2, 1, 0][n tile]: for one kx the tap rows stand in the order
+            // of the accumulators that one strip adds to
             for (int cc = 0; cc < p.cchunks; ++cc)
-                tma_load_3d(wres + (size_t)cc * 9 * p.tap_bytes, &tmW, wfull, cc * CW, run.n0, 0);
+                for (int tap = 0; tap < 9; ++tap)
+                    tma_load_3d(wres + (size_t)(cc * 9 + (tap % 3) * 3 + 2 - tap / 3) * p.tap_bytes, &tmW, wfull,
+                                cc * CW, run.n0, tap);
         }
         __syncwarp();
         uint32_t s = 0, ph = 1, used = 0;
@@ -215,52 +248,54 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
         __syncwarp();
     } else if (warp == 1) {
         // ---- MMA issuer ----
-        const uint32_t idesc = idesc_bf16(128, p.N);
         const uint32_t hi = smem_desc_hi(2 * CW);
         const uint32_t base = smem_u32(smem), w0 = smem_u32(wres);
-        const uint32_t tap16 = p.tap_bytes >> 4;
-        const uint32_t nb1 = (uint32_t)p.nb - 1u;
-        const int nbl = 31 - __clz(p.nb);
-        uint32_t s = 0, ph = 0, li = 0;   // li: output rows opened before this part
+        const uint32_t nb = (uint32_t)p.nb;
+        uint32_t s = 0, ph = 0;
+        uint32_t oslot = 0, ophase = 1;   // the next row to open: its buffer, the parity of the buffer's last release
+        uint32_t cslot = 0;               // the next row to complete
         bool fail = !__all_sync(0xffffffffu, mbar_wait(wfull, 0u, p.err, p.limit_ns));
         for (long long q = run.q0; q < run.q1 && !fail;) {
             const RowSeg g(p, q, run.q1);
             for (int r = g.ha - 1; r <= g.hb && !fail; ++r) {
-                const uint32_t lr = li + (uint32_t)(r - g.ha);   // output row r's place in the ring
+                // output rows r+lo .. r+up (ky = 1-lo .. 1-up) take this strip; the first of
+                // them is in cslot, the last, if r+1, is a new one in oslot
+                const int lo = r > g.ha ? -1 : g.ha - r, up = r + 1 < g.hb ? 1 : g.hb - 1 - r;
+                const bool opens = up == 1, closes = lo == -1;
+                if (opens) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&tempty[oslot], ophase, p.err, p.limit_ns))) {
+                        fail = true;
+                        break;
+                    }
+                    if (++oslot == nb) {
+                        oslot = 0;
+                        ophase ^= 1u;
+                    }
+                }
                 for (int cc = 0; cc < p.cchunks; ++cc) {
                     if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, p.err, p.limit_ns))) {
                         fail = true;
                         break;
                     }
                     tc_fence_after();
-                    const bool four = CW == 64 && (cc + 1 < p.cchunks || p.last_steps == 4);
-                    const uint32_t al = smem_desc_lo(base + s * p.stage_bytes);
-                    const uint32_t bl = smem_desc_lo(w0 + (uint32_t)cc * 9u * p.tap_bytes);
                     if (elect_one()) {
-                        if (r > g.ha) {
-                            const uint32_t j = (lr - 1u) & nb1;
-                            mma_taps<2 * CW>(four, tmem + j * (uint32_t)p.N, al, bl + 6u * tap16, tap16, hi, idesc, true);
-                            if (cc + 1 == p.cchunks) mma_commit(&tfull[j]);
+                        const bool four = CW == 64 && (cc + 1 < p.cchunks || p.last_steps == 4);
+                        const uint32_t al = smem_desc_lo(base + s * p.stage_bytes);
+                        const uint32_t tap16 = p.tap_bytes >> 4;
+                        uint32_t bl = smem_desc_lo(w0 + (uint32_t)cc * 9u * p.tap_bytes) + (uint32_t)(lo + 1) * tap16;
+                        uint32_t slot = cslot;
+                        // as many adjacent accumulators per MMA as N <= 256 and the ring's end allow
+                        for (int left = up - lo + 1; left > 0;) {
+                            const uint32_t c = min((uint32_t)min(left, p.at_once), nb - slot);
+                            left -= (int)c;
+                            mma_rows<2 * CW>(four, tmem + slot * (uint32_t)p.N, (uint32_t)p.N, al, bl, tap16, hi, c,
+                                             opens && cc == 0 && left == 0);
+                            bl += c * tap16;
+                            slot += c;
+                            if (slot == nb) slot = 0;
                         }
-                        if (r >= g.ha && r < g.hb)
-                            mma_taps<2 * CW>(four, tmem + (lr & nb1) * (uint32_t)p.N, al, bl + 3u * tap16, tap16, hi, idesc,
-                                             true);
-                    }
-                    __syncwarp();
-                    const bool opens = r + 1 < g.hb;
-                    const uint32_t lo = lr + 1u;
-                    if (opens && cc == 0 && lo >= (uint32_t)p.nb) {
-                        if (!__all_sync(0xffffffffu, mbar_wait(&tempty[lo & nb1], ((lo >> nbl) - 1u) & 1u, p.err,
-                                                               p.limit_ns))) {
-                            fail = true;
-                            break;
-                        }
-                        tc_fence_after();
-                    }
-                    if (elect_one()) {
-                        if (opens)
-                            mma_taps<2 * CW>(four, tmem + (lo & nb1) * (uint32_t)p.N, al, bl, tap16, hi, idesc, cc != 0);
                         mma_commit(&empty[s]);
+                        if (closes && cc + 1 == p.cchunks) mma_commit(&tfull[cslot]);
                     }
                     __syncwarp();
                     if (++s == (uint32_t)S) {
@@ -268,8 +303,8 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
                         ph ^= 1u;
                     }
                 }
+                if (closes && ++cslot == nb) cslot = 0;
             }
-            li += (uint32_t)(g.hb - g.ha);
             q += g.hb - g.ha;
         }
         // every issued MMA has completed before TMEM is freed
@@ -282,8 +317,7 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
         // ---- epilogue: TMEM lanes 32*(warp % 4) .. +31 are pixels of the row ----
         const int q4 = warp & 3;
         const int row = q4 * 32 + lane;
-        const uint32_t nb1 = (uint32_t)p.nb - 1u;
-        const int nbl = 31 - __clz(p.nb);
+        const uint32_t nb = (uint32_t)p.nb;
         const uint32_t rsw = (uint32_t)((row >> 1) & 3);
         const int grp = (warp - 2) >> 2, bar = 1 + grp;          // the group takes rows grp, grp + 2, ...
         const bool mover = ((warp - 2) & 3) == 0 && elect_one();   // issues the group's copies
@@ -305,9 +339,10 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
         };
         if (EPI == EPI_MASK && mover)
             for (uint32_t k = 0; k + 1 < kTiles && ahead.left > 0; ++k) load_mask();
-        uint32_t li = (uint32_t)grp, j = 0, jph = 0;   // row, its shared tile and that tile's phase
-        for (; cur.left > 0; cur.next(p), cur.next(p), li += 2) {
-            bool ok = mbar_wait(&tfull[li & nb1], (li >> nbl) & 1u, p.err, p.limit_ns);
+        uint32_t slot = (uint32_t)grp, sph = 0;        // the row's accumulator and its phase
+        uint32_t j = 0, jph = 0;                       // its shared tile and that tile's phase
+        for (; cur.left > 0; cur.next(p), cur.next(p)) {
+            bool ok = mbar_wait(&tfull[slot], sph, p.err, p.limit_ns);
             if (EPI == EPI_MASK) {
                 ok = ok && mbar_wait(&gfull[j], jph, p.err, p.limit_ns);
             } else if (mover) {
@@ -318,7 +353,7 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
             if (!epi_and(bar, ok)) break;
             tc_fence_after();
             uint8_t *tile = gio + (size_t)j * p.io_bytes;
-            const uint32_t tbase = tmem + (li & nb1) * (uint32_t)p.N + ((uint32_t)(q4 * 32) << 16);
+            const uint32_t tbase = tmem + slot * (uint32_t)p.N + ((uint32_t)(q4 * 32) << 16);
             for (int c0 = 0; c0 < p.N; c0 += 32) {
                 float v[32];
                 tmem_ld_32x32(tbase + (uint32_t)c0, v);
@@ -358,7 +393,7 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
             // this warp's reads of the accumulator are complete
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[li & nb1]);
+            if (lane == 0) mbar_arrive(&tempty[slot]);
             fence_async_shared();
             epi_sync(bar);
             if (mover) {
@@ -369,6 +404,11 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
                     bulk_wait_read<1>();               // the store before this one has left its tile
                     load_mask();
                 }
+            }
+            slot += 2;
+            if (slot >= nb) {
+                slot -= nb;
+                sph ^= 1u;
             }
             if (++j == kTiles) {
                 j = 0;
@@ -387,7 +427,7 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        tmem_dealloc(tmem, p.tmem_cols);
+        tmem_dealloc(tmem, 512u);
     }
 }
 
@@ -412,14 +452,13 @@ static bool rows_plan(const ConvArgs &c, int epi, RowsParams &p, size_t *smem) {
         p.tap_bytes = (uint32_t)(n * 2 * cw);
         p.w_bytes = p.w_tx = p.cchunks * 9u * p.tap_bytes;
         p.io_bytes = (uint32_t)n * 256u;
-        const size_t fixed = 1024 + p.w_bytes + (size_t)p.nio * p.io_bytes + 8 * (2 * 8 + 2 * 8 + 2 * kTiles + 2) + 16 + 4 * (size_t)n;
+        const size_t fixed = 1024 + p.w_bytes + (size_t)p.nio * p.io_bytes + 8 * (2 * 8 + 2 * 16 + 2 * kTiles + 2) + 16 + 4 * (size_t)n;
         const size_t room = 227u * 1024u;
         if (fixed + 3 * (size_t)p.stage_bytes > room) continue;
         const size_t s = (room - fixed) / p.stage_bytes;
         p.stages = s > 8 ? 8 : (int)s;
-        p.nb = n <= 64 ? 8 : 4;
-        p.tmem_cols = 32;
-        while (p.tmem_cols < (uint32_t)(p.nb * n)) p.tmem_cols <<= 1;
+        p.nb = 512 / n;   // 16, 8, 5 or 4 accumulators in all of TMEM
+        p.at_once = 256 / n < 3 ? 256 / n : 3;
         *smem = fixed + (size_t)p.stages * p.stage_bytes;
         return true;
     }
@@ -462,10 +501,10 @@ cudaError_t conv_rows(const ConvArgs &c, int epi, int *err, unsigned long long l
         const uint32_t b[4] = {bc, bp, 1, 1};
         return tensor_map(m, q, 4, d, s, b, (int)(2 * bc));
     };
-    // w[o][tap*Cin + i] as (i, o, tap): a box of one channel chunk and all taps lands as [tap][o][i]
+    // w[o][tap*Cin + i] as (i, o, tap), a box per channel chunk and tap
     const uint64_t dw[3] = {(uint64_t)c.Cin, (uint64_t)c.Cout, 9};
     const uint64_t sw[2] = {(uint64_t)c.Cin * 18, (uint64_t)c.Cin * 2};
-    const uint32_t bw[3] = {(uint32_t)cw, (uint32_t)p.N, 9};
+    const uint32_t bw[3] = {(uint32_t)cw, (uint32_t)p.N, 1};
     CUtensorMap tx, tw, ty, tm;
     cudaError_t e;
     if ((e = image(&tx, c.x + c.xoff, c.Cin, c.ldx, (uint32_t)cw, 130)) != cudaSuccess) return e;

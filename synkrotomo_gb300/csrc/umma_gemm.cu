@@ -504,9 +504,9 @@ cudaError_t gemm_bf16(const uint16_t *A, const uint16_t *B, float *C, int M, int
 }
 
 // Layers of long rows whose weights do not fit in shared memory beside the
-// strips (192 -> 64 and wider; the others take conv_rows): a tile is 128 pixels of one row, and per input
-// row ky and 64-channel chunk ONE strip of 130 pixels (halo of one on each
-// side) is loaded, with the three taps' weights as one more box; the taps kx
+// strips (192 -> 64 and wider; the others take conv_rows): a tile is 128 pixels
+// of one row, and per input row ky and 64-channel chunk ONE strip of 130 pixels
+// (halo of one on each side) is loaded, with the three taps' weights as one more box; the taps kx
 // are views of the strip shifted by kx rows.  Compared with a box per tap
 // this issues a third of the copy operations and moves a third of the input.
 static cudaError_t conv3x3_halo(const ConvArgs &c, int epi, int ntile, int *err, unsigned long long limit_ns,
