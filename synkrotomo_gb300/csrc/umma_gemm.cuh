@@ -57,6 +57,17 @@ struct WgradArgs {
     int Cin, Cout, B, H, W, ksplit;
 };
 
+// conv_wgrad.cu: the same from the NHWC tensors, with the bias gradient
+// db[o] += sum_p dz[p][o].
+struct DwArgs {
+    const uint16_t *x;    // [B][H][W][ldx], channels xoff .. xoff+Cin-1
+    int ldx, xoff, Cin;
+    const uint16_t *dz;   // [B][H][W][Cout]
+    int Cout, B, H, W;
+    float *dw, *db;       // [Cout][9*Cin], [Cout], accumulated
+};
+cudaError_t conv_wgrad(const DwArgs &a, int *err, unsigned long long limit_ns, cudaStream_t st);
+
 cudaError_t gemm_bf16(const uint16_t *A, const uint16_t *B, float *C, int M, int N, int K, int *err,
                       unsigned long long limit_ns, cudaStream_t st);
 cudaError_t conv3x3(const ConvArgs &c, int epi, int *err, unsigned long long limit_ns, cudaStream_t st);

@@ -48,7 +48,7 @@ struct Net {
     float *params = nullptr, *grads = nullptr, *m = nullptr, *v = nullptr;
     // activations (BF16 NHWC); level l has side N >> l
     uint16_t *e1a, *cat1, *p1, *e2a, *cat2, *p2, *e3a, *cat3, *p3, *e4a, *e4, *d3a, *d3, *d2a, *d2, *d1a, *d1;
-    uint16_t *gA[4], *gB[4], *gcat1, *gcat2, *gcat3, *dzT, *xT3;
+    uint16_t *gA[4], *gB[4], *gcat1, *gcat2, *gcat3;
     float *x0, *tgt, *g;
     double *loss;
     std::vector<void *> allocs;
@@ -136,15 +136,6 @@ cudaError_t net_create(Net **out, int maxB, int N, unsigned long long seed, cuda
     A(n->gcat1, P0 * 96);
     A(n->gcat2, P1 * 192);
     A(n->gcat3, P2 * 384);
-    // channel-major scratch of the weight gradient: largest C*P of any layer
-    size_t dz_max = 0, x_max = 0;
-    for (int l = 1; l < 14; ++l) {
-        const size_t P = Pl[kLevel[l]];
-        dz_max = dz_max > P * kCout[l] ? dz_max : P * kCout[l];
-        x_max = x_max > 3 * P * kCin[l] ? x_max : 3 * P * kCin[l];
-    }
-    A(n->dzT, dz_max);
-    A(n->xT3, x_max);
     A(n->x0, P0);
     A(n->tgt, P0);
     A(n->g, P0);
@@ -248,18 +239,8 @@ static cudaError_t layer_bwd(Net *n, int l, int B, const uint16_t *x, int ldx, i
                              uint16_t *dx, int *err, unsigned long long lim, cudaStream_t st) {
     const Layer &L = n->L[l];
     const int S = n->N >> kLevel[l];
-    const long long P = (long long)B * S * S;
-    NET_TRY(bias_grad(dz, L.cout, n->grads + L.boff, P, L.cout, st));
-    NET_TRY(to_cmajor(dz, L.cout, 0, n->dzT, L.cout, P, S, 0, st));
-    NET_TRY(to_cmajor(x, ldx, xoff, n->xT3, L.cin, P, S, 1, st));
-    const int mt = (L.cout + 127) / 128;
-    const int nt = L.cin <= 256 ? 1 : L.cin / (L.cin % 192 == 0 ? 192 : 128);
-    const long long chunks = P / (S >= 64 ? 64 : 32);
-    long long ks = (152LL * 2) / (9LL * mt * nt);
-    if (ks < 1) ks = 1;
-    if (ks > chunks) ks = chunks;
-    WgradArgs w = {n->dzT, n->xT3, n->grads + L.woff, L.cin, L.cout, B, S, S, (int)ks};
-    NET_TRY(conv3x3_wgrad(w, err, lim, st));
+    DwArgs w = {x, ldx, xoff, L.cin, dz, L.cout, B, S, S, n->grads + L.woff, n->grads + L.boff};
+    NET_TRY(conv_wgrad(w, err, lim, st));
     if (dx) {
         ConvArgs c = {dz, L.cout, 0, L.cout, B, S, S, L.wtbf, nullptr, dx, L.cin, 0, L.cin, x, ldx, xoff};
         NET_TRY(conv3x3(c, EPI_MASK, err, lim, st));

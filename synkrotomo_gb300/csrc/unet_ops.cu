@@ -1,8 +1,7 @@
 // CUDA-core kernels around the tcgen05 convolutions of the U-Net warm
 // starter: the 1-channel input layer, 2x2 max pooling, 2x nearest
 // upsampling into concatenation buffers, the 1x1 output head with the MSE
-// loss, channel-major (transposed, W-shifted) copies for the weight gradient,
-// bias gradients and the fused Adam update.  Activations are BF16 NHWC with a
+// loss and the fused Adam update.  Activations are BF16 NHWC with a
 // channel stride `ld` (so a tensor can be a channel slice of a wider buffer).
 #include <cuda_bf16.h>
 
@@ -312,87 +311,6 @@ __global__ void __launch_bounds__(256) head_bwd_kernel(const float *__restrict__
     }
 }
 
-// Blocked copies for the weight gradient: pixel chunks of cw pixels of one
-// image row (cw = 64 when W >= 64, else 32), each chunk stored as [C][cw].
-// shifted = 0: out[q][c][j] = in[q*cw + j][c] (one copy); shifted = 1: three
-// copies, copy k at k*P*C, holding in[p + k - 1][c] when pixel p+k-1 is in
-// p's image row (w+k-1 in [0, W)), else 0.  A block handles 128 pixels (plus
-// one halo pixel on each side) x 64 channels: 16-byte loads into a
-// channel-major shared tile, then 16-byte stores of 8 consecutive pixels of
-// one channel, so each warp writes whole 128-byte lines.
-__global__ void __launch_bounds__(256) to_cmajor_kernel(const uint16_t *__restrict__ in, int ldi, int ioff,
-                                                        uint16_t *__restrict__ out, int C, long long P, int W,
-                                                        int shifted) {
-    __shared__ uint16_t tile[64][130];   // [channel][pixel p0-1 .. p0+128]; 65-word rows
-    const long long p0 = (long long)blockIdx.x * 128;
-    const int c0 = blockIdx.y * 64;
-    const int cn = min(64, C - c0);      // multiple of 8
-    const int G = cn / 8;
-    const int cw = W >= 64 ? 64 : 32;
-    for (int i = threadIdx.x; i < 130 * G; i += blockDim.x) {
-        const int r = i / G, h = i - r * G;
-        const long long p = p0 - 1 + r;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (p >= 0 && p < P) v = ld8(in + p * ldi + ioff + c0 + 8 * h);
-        const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int k = 0; k < 8; ++k) tile[8 * h + k][r] = (uint16_t)((k & 1) ? (wv[k >> 1] >> 16) : (wv[k >> 1] & 0xffffu));
-    }
-    __syncthreads();
-    const int ncopies = shifted ? 3 : 1;
-    // thread = (channel c, group g of 8 pixels); groups fastest
-    for (int i = threadIdx.x; i < 16 * cn; i += blockDim.x) {
-        const int g = i & 15, c = i >> 4;
-        const long long p = p0 + 8 * g;
-        if (p >= P) continue;            // P is a multiple of 8: a group is wholly in or out
-        const int w0 = (int)(p % W);     // the group lies in one image row (W multiple of 8)
-        const long long q = p / cw;
-        const int j = (int)(p - q * cw);
-        for (int k = 0; k < ncopies; ++k) {
-            const int dsh = shifted ? k - 1 : 0;
-            uint32_t wv[4];
-#pragma unroll
-            for (int e = 0; e < 8; e += 2) {
-                const bool in0 = w0 + e + dsh >= 0 && w0 + e + dsh < W;
-                const bool in1 = w0 + e + 1 + dsh >= 0 && w0 + e + 1 + dsh < W;
-                const uint32_t v0 = in0 ? tile[c][8 * g + e + 1 + dsh] : 0u;
-                const uint32_t v1 = in1 ? tile[c][8 * g + e + 2 + dsh] : 0u;
-                wv[e >> 1] = v0 | (v1 << 16);
-            }
-            uint16_t *o = out + (long long)k * P * C + (q * C + c0 + c) * cw + j;
-            *reinterpret_cast<uint4 *>(o) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-        }
-    }
-}
-
-// db[c] += sum_p dz[p][c].  Thread = (channel group g of 8, pixel lane): a block
-// covers G = C/8 groups x 256/G pixel lanes, 16-byte loads; lanes of one
-// group are summed in shared memory, one atomic per channel per block.
-__global__ void __launch_bounds__(256) bias_grad_kernel(const uint16_t *__restrict__ dz, int ldz,
-                                                        float *__restrict__ db, long long P, int C) {
-    const int G = C / 8;
-    const int lanes = blockDim.x / G;                  // pixel lanes per block
-    const int g = threadIdx.x % G, pl = threadIdx.x / G;
-    float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    if (pl < lanes)
-        for (long long p = (long long)blockIdx.x * lanes + pl; p < P; p += (long long)gridDim.x * lanes) {
-            float v[8];
-            unpack8(ld8(dz + p * ldz + 8 * g), v);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[j] += v[j];
-        }
-    __shared__ float sh[256][9];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) sh[threadIdx.x][j] = pl < lanes ? acc[j] : 0.0f;
-    __syncthreads();
-    for (int c = threadIdx.x; c < C; c += blockDim.x) {
-        const int gg = c / 8, j = c % 8;
-        float t = 0.0f;
-        for (int l = 0; l < lanes; ++l) t += sh[l * G + gg][j];
-        atomicAdd(db + c, t);
-    }
-}
-
 // Fused Adam (bias-corrected): per parameter, g -> m, v -> w; the gradient is
 // zeroed for the next step.  For 3x3 weights [Cout][9][Cin] the BF16 copy and
 // the tap-flipped transposed BF16 copy [Cin][9][Cout] of the backward-data
@@ -491,19 +409,6 @@ cudaError_t head_bwd(const float *g, const uint16_t *d, int ldd, const float *wh
                      float *dbh, long long P, int C, cudaStream_t st) {
     if (C != 32 || !v8(ldd) || !v8(ldz)) return cudaErrorInvalidValue;
     head_bwd_kernel<<<152 * 4, 256, 0, st>>>(g, d, ldd, wh, dz, ldz, dwh, dbh, P, C);
-    return cudaGetLastError();
-}
-cudaError_t to_cmajor(const uint16_t *in, int ldi, int ioff, uint16_t *out, int C, long long P, int W, int shifted,
-                      cudaStream_t st) {
-    if (!v8(C) || !v8(ldi) || !v8(ioff) || W < 32 || W % (W >= 64 ? 64 : 32) || P % W)
-        return cudaErrorInvalidValue;
-    dim3 grid((unsigned)((P + 127) / 128), (unsigned)((C + 63) / 64));
-    to_cmajor_kernel<<<grid, 256, 0, st>>>(in, ldi, ioff, out, C, P, W, shifted);
-    return cudaGetLastError();
-}
-cudaError_t bias_grad(const uint16_t *dz, int ldz, float *db, long long P, int C, cudaStream_t st) {
-    if (!v8(C) || C > 2048 || !v8(ldz)) return cudaErrorInvalidValue;
-    bias_grad_kernel<<<152 * 2, 256, 0, st>>>(dz, ldz, db, P, C);
     return cudaGetLastError();
 }
 cudaError_t adam(float *w, float *g, float *m, float *v, long long n, float lr, float b1, float b2, float eps, int step,

@@ -23,9 +23,6 @@ cudaError_t head(const float *x0, const uint16_t *d, int ldd, const float *wh, c
                  const float *target, float *g, double *loss, long long P, int C, cudaStream_t st);
 cudaError_t head_bwd(const float *g, const uint16_t *d, int ldd, const float *wh, uint16_t *dz, int ldz, float *dwh,
                      float *dbh, long long P, int C, cudaStream_t st);
-cudaError_t to_cmajor(const uint16_t *in, int ldi, int ioff, uint16_t *out, int C, long long P, int W, int shifted,
-                      cudaStream_t st);
-cudaError_t bias_grad(const uint16_t *dz, int ldz, float *db, long long P, int C, cudaStream_t st);
 cudaError_t adam(float *w, float *g, float *m, float *v, long long n, float lr, float b1, float b2, float eps, int step,
                  uint16_t *wbf, uint16_t *wtbf, int Cout, int Cin, cudaStream_t st);
 cudaError_t weights_bf16(const float *w, long long n, uint16_t *wbf, uint16_t *wtbf, int Cout, int Cin,
