@@ -291,13 +291,18 @@ __global__ void __launch_bounds__(192, 1) conv_wgrad_kernel(const __grid_constan
                 const int kx = CI == 64 ? (int)(cm % kM) * 2 + m / 64 : m / 32;   // uniform over the warp
                 if (kx > 2) continue;
                 float *o = p.dw + (long long)co0 * 9 * p.Cin + kx * p.Cin + ci0 + (int)(cm / kM) * CI + m % CI;
-                for (uint32_t n = 0; n < 3u * CO; n += 32u) {
-                    float v[32];
-                    tmem_ld_32x32(tl + cm * 3u * CO + n, v);
-                    const uint32_t ky = 2u - n / CO, oc = n % CO;
+                // groups of 8 columns, each CTA from another one on: in step, all CTAs would
+                // queue at one address after the other
+                constexpr uint32_t kGroups = 3u * CO / 8u;
+                uint32_t g = (uint32_t)part % kGroups;
+                for (uint32_t k = 0; k < kGroups; ++k) {
+                    float v[8];
+                    tmem_ld_32x8(tl + cm * 3u * CO + 8u * g, v);
+                    const uint32_t ky = 2u - 8u * g / CO, oc = 8u * g % CO;
                     float *on = o + (long long)oc * 9 * p.Cin + (long long)ky * 3 * p.Cin;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) atomicAdd(on + (long long)j * 9 * p.Cin, v[j]);
+                    for (int j = 0; j < 8; ++j) atomicAdd(on + (long long)j * 9 * p.Cin, v[j]);
+                    if (++g == kGroups) g = 0;
                 }
             }
             if (t + 1 < p.turns) {
@@ -371,9 +376,13 @@ cudaError_t conv_wgrad(const DwArgs &a, int *err, unsigned long long limit_ns, c
     // one row further than the strip for the atom that is not used
     p.x_bytes = (p.x_tx + 2 * ci + 1023) / 1024 * 1024;
     p.z_bytes = (p.z_tx + 1023) / 1024 * 1024;
-    p.sz = 6;
-    const size_t left = 220u * 1024u - (size_t)p.sz * p.z_bytes;
-    p.sx = left / p.x_bytes < 8 ? (int)(left / p.x_bytes) : 8;
+    // A gradient strip stays for three input rows, so its ring is three strips longer
+    // for the same distance of prefetch.
+    const size_t row = (size_t)p.nc * p.x_bytes + p.z_bytes;
+    size_t depth = (220u * 1024u - 3 * (size_t)p.z_bytes) / row;
+    if (depth > 16) depth = 16;
+    p.sx = (int)depth * p.nc;
+    p.sz = (int)depth + 3;
     p.dw = a.dw;
     p.db = a.db;
     p.err = err;
