@@ -17,11 +17,15 @@
 // shared memory by the warps that later drain the accumulators (FP32 atomics, 32
 // consecutive input channels per instruction).  Pixel rows are split over CTAs.
 //
+// What bounds it: the issuing warp (about 500 cycles per stage for its wait and
+// commit, 35 to 48 per MMA) next to the MMA rate (M=128, N=192: 96 cycles; N=96: 56),
+// and at one image the drain, 10 us of atomics.
 // Against copies of both operands in a channel-major layout (x three times, shifted
 // by kx), one tap per CTA, and a kernel for the bias, 32 images: 32 -> 32 at
-// 256 x 256 448 -> 96 us, 96 -> 32 790 -> 252, 192 -> 64 at 128 x 128 396 -> 111,
-// 384 -> 128 at 64 x 64 237 -> 153, 256 -> 256 at 32 x 32 113 -> 85; the training
-// step 5.98 -> 3.64 ms.
+// 256 x 256 448 -> 191 us, 96 -> 32 790 -> 195, 192 -> 64 at 128 x 128 396 -> 99,
+// 384 -> 128 at 64 x 64 237 -> 104, 256 -> 256 at 32 x 32 113 -> 47; the training
+// step 5.98 -> 3.60 ms.  One row per stage with a barrier per operand and ring:
+// 384 -> 128 149, 256 -> 256 83.
 #include "synk_internal.cuh"
 #include "umma.cuh"
 #include "umma_gemm.cuh"
@@ -32,12 +36,28 @@ namespace unet {
 using namespace umma;
 
 struct DwParams {
-    int Cin, Cout, H, tiles_w, px, nci, nco, nc, splits, turns, sx, sz;
-    long long rows;                    // B * tiles_w * H rows of px pixels
-    uint32_t x_bytes, z_bytes, x_tx, z_tx;
+    int Cin, Cout, H, tiles_w, nci, nco, nc, splits, turns, stages;
+    long long rows;                    // B * tiles_w * H rows of one strip's width
+    uint32_t x_bytes, x_tx, z_tx;      // of one input block's rows in a stage; what a stage's copies bring
     float *dw, *db;
     int *err;
     unsigned long long limit_ns;
+};
+
+// Rows [ha, hb) of one column: a part of a CTA's run.
+struct DwSeg {
+    int b, w0, ha, hb, steps;
+    template <int PX, int R>
+    static __device__ __forceinline__ DwSeg at(const DwParams &p, long long q, long long q1) {
+        DwSeg g;
+        const long long col = q / p.H;
+        g.ha = (int)(q - col * p.H);
+        g.hb = q1 - q < (long long)(p.H - g.ha) ? g.ha + (int)(q1 - q) : p.H;
+        g.b = (int)(col / p.tiles_w);
+        g.w0 = (int)(col - (long long)g.b * p.tiles_w) * PX;
+        g.steps = (g.hb - g.ha + 2 + R - 1) / R;   // input rows ha-1 .. hb, R per step
+        return g;
+    }
 };
 
 __device__ __forceinline__ void tmem_zero32(uint32_t taddr) {
@@ -56,20 +76,24 @@ __device__ __forceinline__ uint32_t desc_lo_mn(uint32_t saddr, uint32_t lead_byt
     return ((saddr & 0x3FFFFu) >> 4) | ((lead_bytes >> 4) << 16);
 }
 
-template <int CI, int CO>
+// KS: K steps of 16 pixels per row (strips of 16 KS pixels); R: image rows per stage.
+template <int CI, int CO, int KS, int R>
 __global__ void __launch_bounds__(192, 1) conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmX,
                                                             const __grid_constant__ CUtensorMap tmZ, const DwParams p) {
+    constexpr int PX = 16 * KS;
     constexpr uint32_t kRowX = 2 * CI, kRowZ = 2 * CO;   // bytes of one pixel
+    constexpr uint32_t kStripX = (PX + 2) * kRowX, kStripZ = PX * kRowZ;
     constexpr uint32_t kM = CI == 64 ? 2 : 1;            // MMAs of M = 128 that hold the three taps kx
+    constexpr int kLate = (2 + R - 1) / R;               // steps for which a gradient row is used again
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *zs = smem_raw + (((raw + 1023u) & ~1023u) - raw);
-    uint8_t *xs = zs + (size_t)p.sz * p.z_bytes;
-    uint64_t *xfull = reinterpret_cast<uint64_t *>(xs + (size_t)p.sx * p.x_bytes);
-    uint64_t *xempty = xfull + p.sx;
-    uint64_t *zfull = xempty + p.sx;
-    uint64_t *zempty = zfull + p.sz;
-    uint64_t *tfull = zempty + p.sz;
+    const int S = p.stages;
+    uint8_t *xs = zs + (size_t)S * R * kStripZ;
+    const uint32_t x_stage = (uint32_t)p.nc * p.x_bytes;
+    uint64_t *full = reinterpret_cast<uint64_t *>(xs + (size_t)S * x_stage);
+    uint64_t *done = full + S;
+    uint64_t *tfull = done + S;
     uint64_t *tempty = tfull + 1;
     uint64_t *drain = tempty + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
@@ -86,13 +110,9 @@ __global__ void __launch_bounds__(192, 1) conv_wgrad_kernel(const __grid_constan
         tmem_relinquish();
     }
     if (warp == 1 && lane == 0) {
-        for (int s = 0; s < p.sx; ++s) {
-            mbar_init(&xfull[s], 1);
-            mbar_init(&xempty[s], 1);
-        }
-        for (int s = 0; s < p.sz; ++s) {
-            mbar_init(&zfull[s], 1);
-            mbar_init(&zempty[s], bias ? 5 : 1);
+        for (int s = 0; s < S; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&done[s], bias ? 5 : 1);   // the step's MMAs, and the four warps of the bias
         }
         mbar_init(tfull, 1);
         mbar_init(tempty, 4);
@@ -107,7 +127,8 @@ __global__ void __launch_bounds__(192, 1) conv_wgrad_kernel(const __grid_constan
     const uint32_t tmem = *tmem_slot;
     constexpr uint32_t kCols = kM * 3u * CO;   // of one input block
     if (warp >= 2) {
-        for (uint32_t c = 0; c < (uint32_t)p.nc * kCols; c += 32u) tmem_zero32(tmem + c + ((uint32_t)((warp & 3) * 32) << 16));
+        for (uint32_t c = 0; c < (uint32_t)p.nc * kCols; c += 32u)
+            tmem_zero32(tmem + c + ((uint32_t)((warp & 3) * 32) << 16));
         tmem_wait_st();
     }
     tc_fence_before();
@@ -115,64 +136,59 @@ __global__ void __launch_bounds__(192, 1) conv_wgrad_kernel(const __grid_constan
     tc_fence_after();
 
     if (warp == 0) {
-        // ---- producer: gradient row r + 1, then the strips of input row r ----
-        uint32_t s = 0, ph = 1, used = 0, zsl = 0, zph = 1, zused = 0;
+        // ---- producer: step i brings input rows r .. r+R-1 and gradient rows r+1 .. r+R,
+        // which the next kLate steps use again: its stage is free when step i + kLate is done ----
+        uint32_t s = 0, used = 0, ph = 0;   // stage; stages filled at least once; parity of this round's "full"
+        uint32_t ws = 0, wph = 0;           // the step to wait for
         bool fail = false;
         for (int t = 0; t < p.turns; ++t)
             for (long long q = q0 + len * t / p.turns, q1 = q0 + len * (t + 1) / p.turns; q < q1 && !fail;) {
-                const long long col = q / p.H;
-                const int ha = (int)(q - col * p.H);
-                const int hb = q1 - q < (long long)(p.H - ha) ? ha + (int)(q1 - q) : p.H;
-                const int b = (int)(col / p.tiles_w), w0 = (int)(col - (long long)b * p.tiles_w) * p.px;
-                for (int r = ha - 1; r <= hb && !fail; ++r) {
-                    if (r + 1 < hb) {
-                        if (!__all_sync(0xffffffffu, mbar_wait(&zempty[zsl], zph, p.err, p.limit_ns))) {
+                const DwSeg g = DwSeg::at<PX, R>(p, q, q1);
+                for (int i = 0; i < g.steps; ++i) {
+                    if (used == (uint32_t)S) {   // the stage was filled before
+                        // step (this one - S + kLate)
+                        if (!__all_sync(0xffffffffu, mbar_wait(&done[ws], wph, p.err, p.limit_ns))) {
                             fail = true;
                             break;
                         }
-                        if (elect_one()) {
-                            mbar_arrive_expect_tx(&zfull[zsl], p.z_tx);
-                            tma_load_4d(zs + (size_t)zsl * p.z_bytes, &tmZ, &zfull[zsl], co0, w0, r + 1, b);
-                        }
-                        __syncwarp();
-                        if (zused < (uint32_t)p.sz) ++zused;
-                        if (++zsl == (uint32_t)p.sz) {
-                            zsl = 0;
-                            zph ^= 1u;
+                        if (++ws == (uint32_t)S) {
+                            ws = 0;
+                            wph ^= 1u;
                         }
                     }
-                    for (int c = 0; c < p.nc; ++c) {
-                        if (!__all_sync(0xffffffffu, mbar_wait(&xempty[s], ph, p.err, p.limit_ns))) {
-                            fail = true;
-                            break;
-                        }
-                        if (elect_one()) {
-                            // rows -1 and H and pixels -1 and W are out of bounds and read as 0
-                            mbar_arrive_expect_tx(&xfull[s], p.x_tx);
-                            tma_load_4d(xs + (size_t)s * p.x_bytes, &tmX, &xfull[s], ci0 + c * CI, w0 - 1, r, b);
-                        }
-                        __syncwarp();
-                        if (used < (uint32_t)p.sx) ++used;
-                        if (++s == (uint32_t)p.sx) {
-                            s = 0;
-                            ph ^= 1u;
-                        }
+                    if (elect_one()) {
+                        const int r = g.ha - 1 + i * R;
+                        const bool z = r + 1 < g.hb;
+                        // rows and pixels outside the image read as 0
+                        mbar_arrive_expect_tx(&full[s], (uint32_t)p.nc * p.x_tx + (z ? p.z_tx : 0u));
+                        if (z) tma_load_4d(zs + (size_t)s * R * kStripZ, &tmZ, &full[s], co0, g.w0, r + 1, g.b);
+                        for (int c = 0; c < p.nc; ++c)
+                            tma_load_4d(xs + (size_t)s * x_stage + (size_t)c * p.x_bytes, &tmX, &full[s], ci0 + c * CI,
+                                        g.w0 - 1, r, g.b);
+                    }
+                    __syncwarp();
+                    if (used < (uint32_t)S && ++used == (uint32_t)S) {
+                        ws = (uint32_t)kLate;   // the first wait is for step kLate
+                        wph = 0;
+                    }
+                    if (++s == (uint32_t)S) {
+                        s = 0;
+                        ph ^= 1u;
                     }
                 }
-                q += hb - ha;
+                q += g.hb - g.ha;
             }
-        // no copy may still be landing when the CTA exits
-        for (uint32_t c = 0; c < used; ++c) mbar_drain(&xfull[c], c < s ? ph ^ 1u : ph, p.limit_ns);
-        for (uint32_t c = 0; c < zused; ++c) mbar_drain(&zfull[c], c < zsl ? zph ^ 1u : zph, p.limit_ns);
+        // no copy may still be landing when the CTA exits: stages below s were last
+        // filled in this round, the others in the one before
+        for (uint32_t c = 0; c < used; ++c) mbar_drain(&full[c], c < s ? ph : ph ^ 1u, p.limit_ns);
         __syncwarp();
     } else if (warp == 1) {
         // ---- MMA issuer ----
         const uint32_t xhi = smem_desc_hi(kRowX), zhi = smem_desc_hi(kRowZ);
         const uint32_t x0 = smem_u32(xs), z0 = smem_u32(zs);
         const uint32_t id1 = idesc_bf16(128, 0) | (3u << 15);   // both operands MN-major
-        const uint32_t sz = (uint32_t)p.sz;
-        const int ksteps = p.px / 16;
-        uint32_t s = 0, ph = 0, osl = 0, oph = 0, csl = 0;
+        const uint32_t zrows = (uint32_t)(S * R);
+        uint32_t s = 0, ph = 0;
         bool fail = false;
         for (int t = 0; t < p.turns && !fail; ++t) {
             if (t > 0) {
@@ -181,60 +197,55 @@ __global__ void __launch_bounds__(192, 1) conv_wgrad_kernel(const __grid_constan
             }
             const long long q1 = q0 + len * (t + 1) / p.turns;
             for (long long q = q0 + len * t / p.turns; q < q1 && !fail;) {
-                const long long col = q / p.H;
-                const int ha = (int)(q - col * p.H);
-                const int hb = q1 - q < (long long)(p.H - ha) ? ha + (int)(q1 - q) : p.H;
-                for (int r = ha - 1; r <= hb; ++r) {
-                    // gradient rows r+lo .. r+up (ky = 1-lo .. 1-up) meet this input row; the
-                    // first is in ring slot csl
-                    const int lo = r > ha ? -1 : ha - r, up = r + 1 < hb ? 1 : hb - 1 - r;
-                    const bool closes = lo == -1;
-                    if (up == 1) {
-                        if (!__all_sync(0xffffffffu, mbar_wait(&zfull[osl], oph, p.err, p.limit_ns))) fail = true;
-                        if (++osl == sz) {
-                            osl = 0;
-                            oph ^= 1u;
-                        }
+                const DwSeg g = DwSeg::at<PX, R>(p, q, q1);
+                uint32_t zsl = s * R;   // ring slot of the first gradient row that meets input row r
+                for (int i = 0; i < g.steps; ++i) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, p.err, p.limit_ns))) {
+                        fail = true;
+                        break;
                     }
-                    for (int c = 0; c < p.nc && !fail; ++c) {
-                        if (!__all_sync(0xffffffffu, mbar_wait(&xfull[s], ph, p.err, p.limit_ns))) {
-                            fail = true;
-                            break;
-                        }
-                        tc_fence_after();
+                    tc_fence_after();
+                    const uint32_t xa = x0 + s * x_stage;
+#pragma unroll
+                    for (int j = 0; j < R; ++j) {
+                        // gradient rows r+lo .. r+up (ky = 1-lo .. 1-up) meet input row r
+                        const int r = g.ha - 1 + i * R + j;
+                        const int lo = r > g.ha ? -1 : g.ha - r, up = r + 1 < g.hb ? 1 : g.hb - 1 - r;
+                        if (lo > up) continue;   // past the last row
                         if (elect_one()) {
-                            const uint32_t al = desc_lo_mn(x0 + s * p.x_bytes, kRowX);
-                            uint32_t slot = csl, d = tmem + (uint32_t)c * kCols + (uint32_t)(lo + 1) * CO;
-                            for (int left = up - lo + 1; left > 0;) {
-                                // neighbours in the ring, up to its end
-                                const uint32_t n = min((uint32_t)left, sz - slot);
-                                const uint32_t idn = id1 | ((n * CO >> 3) << 17);
-                                const uint32_t bl = desc_lo_mn(z0 + slot * p.z_bytes, p.z_bytes);
-#pragma unroll 2
-                                for (int k = 0; k < ksteps; ++k) {
-                                    const uint32_t ak = al + (uint32_t)k * kRowX, bk = bl + (uint32_t)k * kRowZ;
-                                    mma_bf16(d, ak, xhi, bk, zhi, idn, 1u);
-                                    if (CI == 64)
-                                        mma_bf16(d + 3u * CO, ak + 2u * (kRowX / 16u), xhi, bk, zhi, idn, 1u);
+                            for (int c = 0; c < p.nc; ++c) {
+                                const uint32_t al = desc_lo_mn(xa + (uint32_t)c * p.x_bytes + (uint32_t)j * kStripX, kRowX);
+                                uint32_t slot = zsl, d = tmem + (uint32_t)c * kCols + (uint32_t)(lo + 1) * CO;
+                                for (int left = up - lo + 1; left > 0;) {
+                                    // neighbours in the ring, up to its end
+                                    const uint32_t n = min((uint32_t)left, zrows - slot);
+                                    const uint32_t idn = id1 | ((n * CO >> 3) << 17);
+                                    const uint32_t bl = desc_lo_mn(z0 + slot * kStripZ, kStripZ);
+#pragma unroll
+                                    for (uint32_t k = 0; k < (uint32_t)KS; ++k) {
+                                        mma_bf16(d, al + k * kRowX, xhi, bl + k * kRowZ, zhi, idn, 1u);
+                                        if (CI == 64)
+                                            mma_bf16(d + 3u * CO, al + k * kRowX + 2u * (kRowX / 16u), xhi,
+                                                     bl + k * kRowZ, zhi, idn, 1u);
+                                    }
+                                    left -= (int)n;
+                                    d += n * CO;
+                                    slot += n;
+                                    if (slot == zrows) slot = 0;
                                 }
-                                left -= (int)n;
-                                d += n * CO;
-                                slot += n;
-                                if (slot == sz) slot = 0;
                             }
-                            mma_commit(&xempty[s]);
-                            if (closes && c + 1 == p.nc) mma_commit(&zempty[csl]);
                         }
                         __syncwarp();
-                        if (++s == (uint32_t)p.sx) {
-                            s = 0;
-                            ph ^= 1u;
-                        }
+                        if (lo == -1 && ++zsl == zrows) zsl = 0;
                     }
-                    if (fail) break;
-                    if (closes && ++csl == sz) csl = 0;
+                    if (elect_one()) mma_commit(&done[s]);
+                    __syncwarp();
+                    if (++s == (uint32_t)S) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
                 }
-                q += hb - ha;
+                q += g.hb - g.ha;
             }
             if (!fail && elect_one()) mma_commit(tfull);   // the sums are signalled only whole
             __syncwarp();
@@ -252,36 +263,44 @@ __global__ void __launch_bounds__(192, 1) conv_wgrad_kernel(const __grid_constan
         // bias: lane = (pixel, 8 channels); a warp takes a quarter of a strip's pixels
         constexpr uint32_t kG = CO / 8, kStep = 32 / kG;
         const uint32_t c = (uint32_t)lane % kG, r0 = (uint32_t)lane / kG;
-        const uint32_t per = (uint32_t)p.px / 4u;
+        constexpr uint32_t kPer = PX / 4u;
         float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        uint32_t zsl = 0, zph = 0;
+        uint32_t s = 0, ph = 0;
         bool ok = true;
         for (int t = 0; t < p.turns && ok; ++t) {
             const long long q1 = q0 + len * (t + 1) / p.turns;
-            for (long long q = bias ? q0 + len * t / p.turns : q1; q < q1; ++q) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&zfull[zsl], zph, p.err, p.limit_ns));
-                if (!ok) break;
-                const uint8_t *z = zs + (size_t)zsl * p.z_bytes;
-                float u8[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-                for (uint32_t i = r0; i < per; i += kStep) {
-                    const uint32_t row = (uint32_t)q4 * per + i;
-                    const uint32_t sw = CO == 64 ? row & 7u : (row >> 1) & 3u;
-                    const uint4 u = *reinterpret_cast<const uint4 *>(z + row * kRowZ + ((c ^ sw) << 4));
-                    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+            for (long long q = bias ? q0 + len * t / p.turns : q1; q < q1 && ok;) {
+                const DwSeg g = DwSeg::at<PX, R>(p, q, q1);
+                for (int i = 0; i < g.steps; ++i) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(&full[s], ph, p.err, p.limit_ns));
+                    if (!ok) break;
+                    const int rows = min(R, g.hb - g.ha - i * R);   // gradient rows of this step
+                    for (int j = 0; j < rows; ++j) {
+                        const uint8_t *z = zs + (size_t)(s * R + (uint32_t)j) * kStripZ;
+                        float u8[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        u8[2 * e] += __uint_as_float(w[e] << 16);
-                        u8[2 * e + 1] += __uint_as_float(w[e] & 0xffff0000u);
+                        for (uint32_t k = 0; k < kPer; k += kStep) {
+                            const uint32_t row = (uint32_t)q4 * kPer + k + r0;
+                            const uint32_t sw = CO == 64 ? row & 7u : (row >> 1) & 3u;
+                            const uint4 u = *reinterpret_cast<const uint4 *>(z + row * kRowZ + ((c ^ sw) << 4));
+                            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                u8[2 * e] += __uint_as_float(w[e] << 16);
+                                u8[2 * e + 1] += __uint_as_float(w[e] & 0xffff0000u);
+                            }
+                        }
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) acc[e] += u8[e];
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&done[s]);
+                    if (++s == (uint32_t)S) {
+                        s = 0;
+                        ph ^= 1u;
                     }
                 }
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc[e] += u8[e];
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&zempty[zsl]);
-                if (++zsl == (uint32_t)p.sz) {
-                    zsl = 0;
-                    zph ^= 1u;
-                }
+                q += g.hb - g.ha;
             }
             ok = __all_sync(0xffffffffu, ok && mbar_wait(tfull, (uint32_t)t & 1u, p.err, p.limit_ns));
             if (!ok) break;
@@ -331,75 +350,78 @@ __global__ void __launch_bounds__(192, 1) conv_wgrad_kernel(const __grid_constan
     }
 }
 
-template <int CI, int CO>
-static cudaError_t dw_launch(const CUtensorMap &x, const CUtensorMap &z, const DwParams &p, size_t smem, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(conv_wgrad_kernel<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    conv_wgrad_kernel<CI, CO><<<(unsigned)(p.nci * p.nco * p.splits), 192, smem, st>>>(x, z, p);
-    return cudaGetLastError();
-}
-
-cudaError_t conv_wgrad(const DwArgs &a, int *err, unsigned long long limit_ns, cudaStream_t st) {
-    if (a.Cin % 32 || a.Cout % 32 || (a.W > 128 ? a.W % 128 : a.W % 16) || a.ldx % 8 || a.xoff % 8)
-        return cudaErrorInvalidValue;
-    // blocks of 64 channels where they divide, else 32
-    const int ci = a.Cin % 64 == 0 ? 64 : 32, co = a.Cout % 64 == 0 ? 64 : 32;
-    DwParams p = {};
-    p.Cin = a.Cin;
-    p.Cout = a.Cout;
-    p.H = a.H;
-    p.px = a.W < 128 ? a.W : 128;
-    p.tiles_w = a.W / p.px;
+template <int CI, int CO, int KS, int R>
+static cudaError_t dw_launch(const DwArgs &a, DwParams &p, cudaStream_t st) {
+    constexpr int PX = 16 * KS;
+    static_assert(PX / 4 % (32 / (CO / 8)) == 0, "a warp's share of a strip is whole steps of the bias sums");
+    p.tiles_w = a.W / PX;
     p.rows = (long long)a.B * p.tiles_w * a.H;
     if (p.rows == 0) return cudaSuccess;
+    const int chunks = a.Cin / CI, cols = (CI == 64 ? 2 : 1) * 3 * CO;
     // While the rows are few a CTA takes as many input blocks as the 512 TMEM columns
-    // hold, so that a gradient strip is read for all of them.  From 8192 rows on it
-    // takes one: three blocks over the 96 input channels of a batch of 32 leave sums
-    // of 864 steps instead of 2624, and the cut-off bits (see below) that are missing
-    // from them then move the gradient by 2.2e-5 of its norm from what sums of 3970
-    // steps, one tap per CTA, gave; with one block it stays within 2e-5.
-    const int chunks = a.Cin / ci, cols = (ci == 64 ? 2 : 1) * 3 * co;
+    // hold, so that a gradient strip is read for all of them, and all SMs work.  The
+    // tensor cores' FP32 sums cut off below their last bit at every step, 2^-25 of
+    // the sum on average.  Where the rows are many (full-resolution layers of 12 and
+    // more images) the cut-off bits that shorter sums do not lose would move the
+    // gradient by up to 2.1e-5 of its norm from what it was with one tap per CTA and
+    // 33 parts (3970 steps a sum at 32 images): there 40 parts of one block each, 3277
+    // steps.
+    const bool many = CI == 32 && CO == 32 && p.rows > 6144;
     p.nc = 1;
-    if (p.rows < 8192)
+    if (!many)
         for (p.nc = 512 / cols < chunks ? 512 / cols : chunks; chunks % p.nc; --p.nc) {}
     p.nci = chunks / p.nc;
-    p.nco = a.Cout / co;
+    p.nco = a.Cout / CO;
     const int nblk = p.nci * p.nco, sms = device_sms();
-    const long long want = nblk < sms ? sms / nblk : 1;
+    long long want = nblk < sms ? sms / nblk : 1;
+    if (many && want > 40) want = 40;
     p.splits = (int)(want < p.rows ? want : p.rows);
-    // the tensor cores' FP32 sums cut off below their last bit at every step: none
-    // covers more than a sixteenth of the pixels before it joins the rounded totals
+    // nor does any sum cover more than a sixteenth of the pixels
     p.turns = (16 + p.splits - 1) / p.splits;
-    p.x_tx = (uint32_t)(p.px + 2) * 2 * ci;
-    p.z_tx = (uint32_t)p.px * 2 * co;
-    // one row further than the strip for the atom that is not used
-    p.x_bytes = (p.x_tx + 2 * ci + 1023) / 1024 * 1024;
-    p.z_bytes = (p.z_tx + 1023) / 1024 * 1024;
-    // A gradient strip stays for three input rows, so its ring is three strips longer
-    // for the same distance of prefetch.
-    const size_t row = (size_t)p.nc * p.x_bytes + p.z_bytes;
-    size_t depth = (220u * 1024u - 3 * (size_t)p.z_bytes) / row;
-    if (depth > 16) depth = 16;
-    p.sx = (int)depth * p.nc;
-    p.sz = (int)depth + 3;
-    p.dw = a.dw;
-    p.db = a.db;
-    p.err = err;
-    p.limit_ns = limit_ns;
-    const size_t smem = 1024 + (size_t)p.sx * p.x_bytes + (size_t)p.sz * p.z_bytes + 8 * (2 * p.sx + 2 * p.sz + 3) + 16;
+    p.x_tx = (uint32_t)(R * (PX + 2) * 2 * CI);
+    p.z_tx = (uint32_t)(R * PX * 2 * CO);
+    // one pixel further than the strips for the atom that is not used
+    p.x_bytes = (p.x_tx + 2 * CI + 1023) / 1024 * 1024;
+    const size_t stage = p.z_tx + (size_t)p.nc * p.x_bytes;
+    p.stages = (int)(220u * 1024u / stage) < 12 ? (int)(220u * 1024u / stage) : 12;
+    const size_t smem = 1024 + p.stages * stage + 8 * (2 * p.stages + 3) + 16;
     CUtensorMap tx, tz;
     auto image = [&](CUtensorMap *m, const uint16_t *q, int ch, int ld, int bc, int bp) {
         const uint64_t d[4] = {(uint64_t)ch, (uint64_t)a.W, (uint64_t)a.H, (uint64_t)a.B};
         const uint64_t s[3] = {(uint64_t)ld * 2, (uint64_t)ld * 2 * a.W, (uint64_t)ld * 2 * a.W * a.H};
-        const uint32_t b[4] = {(uint32_t)bc, (uint32_t)bp, 1, 1};
+        const uint32_t b[4] = {(uint32_t)bc, (uint32_t)bp, (uint32_t)R, 1};
         return tensor_map(m, q, 4, d, s, b, 2 * bc);
     };
     cudaError_t e;
-    if ((e = image(&tx, a.x + a.xoff, a.Cin, a.ldx, ci, p.px + 2)) != cudaSuccess) return e;
-    if ((e = image(&tz, a.dz, a.Cout, a.Cout, co, p.px)) != cudaSuccess) return e;
-    if (ci == 64) return co == 64 ? dw_launch<64, 64>(tx, tz, p, smem, st) : dw_launch<64, 32>(tx, tz, p, smem, st);
-    return co == 64 ? dw_launch<32, 64>(tx, tz, p, smem, st) : dw_launch<32, 32>(tx, tz, p, smem, st);
+    if ((e = image(&tx, a.x + a.xoff, a.Cin, a.ldx, CI, PX + 2)) != cudaSuccess) return e;
+    if ((e = image(&tz, a.dz, a.Cout, a.Cout, CO, PX)) != cudaSuccess) return e;
+    auto kernel = conv_wgrad_kernel<CI, CO, KS, R>;
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+    kernel<<<(unsigned)(nblk * p.splits), 192, smem, st>>>(tx, tz, p);
+    return cudaGetLastError();
+}
+
+cudaError_t conv_wgrad(const DwArgs &a, int *err, unsigned long long limit_ns, cudaStream_t st) {
+    if (a.Cin % 32 || a.Cout % 32 || a.ldx % 8 || a.xoff % 8) return cudaErrorInvalidValue;
+    DwParams p = {};
+    p.Cin = a.Cin;
+    p.Cout = a.Cout;
+    p.H = a.H;
+    p.dw = a.dw;
+    p.db = a.db;
+    p.err = err;
+    p.limit_ns = limit_ns;
+    // Strips of 128 pixels, or the whole of narrower rows, and as many rows per stage as
+    // give its hand-off (a wait, a commit: about 500 cycles of the issuing warp) 16
+    // MMAs to stand against.
+    if (a.Cin % 64 || a.Cout % 64) {
+        if (a.W % 128) return cudaErrorInvalidValue;
+        return a.Cout % 64 == 0 ? dw_launch<32, 64, 8, 2>(a, p, st) : dw_launch<32, 32, 8, 2>(a, p, st);
+    }
+    if (a.W % 128 == 0) return dw_launch<64, 64, 8, 1>(a, p, st);
+    if (a.W == 64) return dw_launch<64, 64, 4, 2>(a, p, st);
+    if (a.W == 32) return dw_launch<64, 64, 2, 4>(a, p, st);
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace unet
