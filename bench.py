@@ -766,7 +766,7 @@ def main():
             "config": bench_config(world),
             "fp_ms": res["fp_ms"], "bp_ms": res["bp_ms"],
             # per step: setup (geometry_kernel when a > 1024, setup_kernel) + fp_lane_kernel + fp_exact_kernel
-            # (FP); setup + row_scale_kernel + bp_tile_kernel (BP)
+            # (FP); setup + row_pair_kernel + bp_tile_kernel (BP)
             "gpu_launches": (2 * (2 if N_ANGLES > 1024 else 1) + 4) * args.steps,
             "clocks": res["clocks"], "roofline": roofline}
     e = res["e2e"]

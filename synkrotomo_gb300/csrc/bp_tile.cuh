@@ -44,7 +44,7 @@ __device__ __forceinline__ void bp_stage(const ProbGeom &P, int k0, BpStage &st)
         float2 l = make_float2(0.0f, -1.0f);
         if (k < P.a) {
             const AngleGeom g = load_geom(P.geom, k);
-            if (!g.exact) {
+            if (!g.exact && isfinite(g.c)) {               // an angle without a direction weighs nothing
                 v = make_float4(g.c, g.s, g.h_over_b, g.inv_b);
                 l = make_float2(g.lbase, fmaf(-(1.0f - fact_f32()), g.inv_b, g.h_over_b));
             }
@@ -150,59 +150,107 @@ __device__ __forceinline__ void bp_chunk(const ProbGeom &P, const BpStage &st, i
     for (; i < nk; i += kstride) angle(i);
 }
 
-// The UNIT, INRANGE, SCALED path on detector pairs: entry s of row k is (row[s],
-// row[s+1]), so one 8-byte gather serves both candidates of a pixel and angle,
-// and one packed multiply-add (acc_0, acc_1) += (w0, w1) * (v0, v1).  Angles kc
-// .. of the staged chunk into out[m] (overwritten).  Two pixels' coordinates,
-// ceilings and fractions are computed at a time with packed instructions (the
-// halves round as the scalar ones), and a gather's address is a 32-bit offset
-// in the chunk's rows (a chunk of 256 in-range rows is below 4 GB): the 64-bit
-// wide multiply-add it replaces holds the FMA pipe for four to five cycles.
+// The same sums on detector pairs: entry pad + s of row k (W entries a row) holds
+// detectors (s, s+1), already times the row's factor and zero outside [0, D), so
+// one 8-byte gather serves two candidates of a pixel and angle, and one packed
+// multiply-add (acc_0, acc_1) += (w0, w1) * (v0, v1).  Angles kphase, kphase +
+// 2^lgstride, ... of the chunk staged from kc on go into out[m] (overwritten).  Two
+// pixels' coordinates, ceilings and distances are computed at a time with packed
+// instructions (the halves round as the scalar ones), and a gather's address is a
+// 32-bit offset in the chunk's rows (the caller keeps 256 rows below 4 GB): the
+// 64-bit wide multiply-add it replaces holds the FMA pipe for four to five cycles.
+// UNIT: deltarho = 1 (bp_chunk's weights); otherwise RPP candidates, at most four.
+// CLAMP: first candidates may lie outside the row's entries; those outside
+// [-pad, D] are moved to its ends, which are zero (PairRows).
 // Two angles at a time with 80 registers (3 blocks per SM), N=2048, 2048 angles:
 // 4.05 -> 3.44 ms (one at a time 4.25; 64 registers 3.75; three with 128 registers
 // 3.62; the tile's segments staged in shared memory 3.88).
-template <int PIX>
+template <int PIX, int RPP = 2, bool UNIT = true, bool CLAMP = false>
 __device__ __forceinline__ void bp_chunk_pair(const ProbGeom &P, const BpStage &st, int kc,
-                                              const float2 *__restrict__ pairs, float xc, float yc0, float ystep,
-                                              float (&out)[PIX]) {
+                                              const float2 *__restrict__ pairs, int W, int pad, int kphase,
+                                              int lgstride, float xc, float yc0, float ystep, float (&out)[PIX]) {
     static_assert(PIX % 2 == 0, "pixels go in pairs");
+    static_assert(!UNIT || RPP == 2, "two candidates at deltarho = 1");
     const float fact = fact_f32();
-    const float zoff = -P.rz_c - fact;
     const f32x2 mg2 = pk2(kMagic, kMagic), nmg2 = pk2(-kMagic, -kMagic), m1 = pk2(-1.0f, -1.0f);
     const f32x2 nf2 = pk2(-fact, -fact);
-    const char *base = reinterpret_cast<const char *>(pairs + (size_t)kc * P.D);
-    const unsigned step = (unsigned)P.D * 8u;
+    // not UNIT: coordinates are kept negated (-q), so that s0*deltarho - q is one multiply-add
+    const f32x2 f2 = pk2(fact, fact), ninv2 = pk2(-P.inv_deltarho, -P.inv_deltarho), dr2 = pk2(P.deltarho, P.deltarho);
+    const char *base = reinterpret_cast<const char *>(pairs + (size_t)kc * W);
+    const unsigned step = ((unsigned)W * 8u) << lgstride;
     // gather offset in the chunk = bits(r)*8 + rowoff (mod 2^32), bits(r) = kMagicBits + s0 - zi
-    unsigned rowoff = ((unsigned)P.zi - (unsigned)kMagicBits) * 8u;
-    const int nk = min(kBpChunk, P.a - kc);
+    unsigned rowoff = ((unsigned)(P.zi + pad) - (unsigned)kMagicBits) * 8u + (unsigned)W * 8u * (unsigned)kphase;
+    // limits of r: the zero entries, or 2^21, which no pixel's window reaches
+    const float rlo = kMagic + (float)max(-pad - P.zi, -(1 << 21));
+    const float rhi = kMagic + (float)min(P.D - P.zi, 1 << 21);
+    const int nk = (min(kBpChunk, P.a - kc) - kphase + (1 << lgstride) - 1) >> lgstride;   // this part's angles
     f32x2 acc[PIX];
 #pragma unroll
     for (int m = 0; m < PIX; ++m) acc[m] = pk2(0.0f, 0.0f);
 #pragma unroll 2
-    for (int i = 0; i < nk; ++i) {
+    for (int j = 0; j < nk; ++j) {
+        const int i = (j << lgstride) + kphase;
         const float4 g = st.cs[i];
-        const float c1 = st.le[i].y;
-        // q of pixel m from the angle's base value in one rounding (see bp_chunk)
-        const float q0 = fmaf(xc, g.x, fmaf(-yc0, g.y, zoff));
-        const float dq = -ystep * g.y;
-        const f32x2 q02 = pk2(q0, q0), dq2 = pk2(dq, dq);
-        float2 v[PIX], w[PIX];
+        auto entry = [&](float r) {
+            if constexpr (CLAMP) r = fminf(fmaxf(r, rlo), rhi);
+            return base + ((unsigned)__float_as_int(r) * 8u + rowoff);
+        };
+        if constexpr (UNIT) {
+            const float c1 = st.le[i].y;
+            // q of pixel m from the angle's base value in one rounding (see bp_chunk)
+            const float q0 = fmaf(xc, g.x, fmaf(-yc0, g.y, -P.rz_c - fact));
+            const float dq = -ystep * g.y;
+            const f32x2 q02 = pk2(q0, q0), dq2 = pk2(dq, dq);
+            float2 v[PIX], w[PIX];
 #pragma unroll
-        for (int h = 0; h < PIX / 2; ++h) {
-            const f32x2 q = fma2(pk2((float)(2 * h), (float)(2 * h + 1)), dq2, q02);
-            const f32x2 r = add2_ru(q, mg2);
-            const f32x2 e = fma2(q, m1, add2(r, nmg2));            // ceil(q) - q
-            const float2 ev = unpk2(e), dv = unpk2(add2(e, nf2)), rv = unpk2(r);
+            for (int h = 0; h < PIX / 2; ++h) {
+                const f32x2 q = fma2(pk2((float)(2 * h), (float)(2 * h + 1)), dq2, q02);
+                const f32x2 r = add2_ru(q, mg2);
+                const f32x2 e = fma2(q, m1, add2(r, nmg2));            // ceil(q) - q
+                const float2 ev = unpk2(e), dv = unpk2(add2(e, nf2)), rv = unpk2(r);
 #pragma unroll
-            for (int o = 0; o < 2; ++o) {
-                v[2 * h + o] = __ldg(reinterpret_cast<const float2 *>(
-                    base + ((unsigned)__float_as_int(o ? rv.y : rv.x) * 8u + rowoff)));
-                w[2 * h + o].x = __saturatef(fmaf(-fabsf(o ? dv.y : dv.x), g.w, g.z));
-                w[2 * h + o].y = __saturatef(fmaf(-(o ? ev.y : ev.x), g.w, c1));
+                for (int o = 0; o < 2; ++o) {
+                    v[2 * h + o] = __ldg(reinterpret_cast<const float2 *>(entry(o ? rv.y : rv.x)));
+                    w[2 * h + o].x = __saturatef(fmaf(-fabsf(o ? dv.y : dv.x), g.w, g.z));
+                    w[2 * h + o].y = __saturatef(fmaf(-(o ? ev.y : ev.x), g.w, c1));
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < PIX; ++m) acc[m] = fma2(pk2(w[m]), pk2(v[m]), acc[m]);
+        } else {
+            const float nt0 = fmaf(yc0, g.y, P.rz_c), dt = ystep * g.y;   // -(rho - rz_c) = -x*cos + y*sin + rz_c
+            const f32x2 nc2 = pk2(-g.x, -g.x), xc2 = pk2(xc, xc), nt02 = pk2(nt0, nt0), dt2 = pk2(dt, dt);
+#pragma unroll
+            for (int h = 0; h < PIX / 2; ++h) {
+                const f32x2 t = fma2(pk2((float)(2 * h), (float)(2 * h + 1)), dt2, nt02);
+                const f32x2 nq = fma2(xc2, nc2, t);
+                const f32x2 r = add2_ru(mul2(add2(nq, f2), ninv2), mg2);
+                const float2 rv = unpk2(r);
+                const char *p[2] = {entry(rv.x), entry(rv.y)};
+                f32x2 d = fma2(add2(r, nmg2), dr2, nq);                  // distance of the first candidate
+#pragma unroll
+                for (int c = 0; c < RPP; c += 2) {
+                    const float2 d0 = unpk2(d);
+                    d = add2(d, dr2);
+                    const float2 d1 = unpk2(d);
+                    d = add2(d, dr2);
+#pragma unroll
+                    for (int o = 0; o < 2; ++o) {
+                        const float w0 = __saturatef(fmaf(-fabsf(o ? d0.y : d0.x), g.w, g.z));
+                        if (c + 1 < RPP) {
+                            const float w1 = __saturatef(fmaf(-fabsf(o ? d1.y : d1.x), g.w, g.z));
+                            const float2 v = __ldg(reinterpret_cast<const float2 *>(p[o] + c * 8));
+                            acc[2 * h + o] = fma2(pk2(w0, w1), pk2(v), acc[2 * h + o]);
+                        } else {
+                            const float v = __ldg(reinterpret_cast<const float *>(p[o] + c * 8));
+                            float2 a = unpk2(acc[2 * h + o]);
+                            a.x = fmaf(w0, v, a.x);
+                            acc[2 * h + o] = pk2(a);
+                        }
+                    }
+                }
             }
         }
-#pragma unroll
-        for (int m = 0; m < PIX; ++m) acc[m] = fma2(pk2(w[m]), pk2(v[m]), acc[m]);
         rowoff += step;
     }
 #pragma unroll
@@ -237,6 +285,36 @@ inline bool bp_windows_in_range(const ProbGeom &P, int tile_rows) {
     const double margin = 1e-2 + 1e-5 * (R + fabs(rz));
     const double lo = -R - f - rz, hi = R - f - rz;
     return ceil(lo - margin) >= 0.0 && ceil(hi + margin) + 1.0 <= (double)P.D - 1.0;
+}
+
+// Rows of bp_chunk_pair: `pad` zero entries before detector 0, W = D + 2*pad - 1
+// entries.  A first candidate s has its entries when -pad <= s <= D + pad - 2 (two
+// less with a second pair).
+struct PairRows {
+    int pad, W;
+    bool inrange;    // every tile pixel's first candidate has its entries: no CLAMP
+};
+
+// The pixels of a tile past the image's edge reach up to 63*sqrt(2) further than
+// the image, so the rows are padded as far as they need (at most kBpMaxPad,
+// else CLAMP, which costs a minimum and a maximum per gather: N=2046, 1999 angles
+// 4.28 ms with it, 3.37 without).
+constexpr int kBpMaxPad = 128;
+inline PairRows bp_pair_rows(const ProbGeom &P, int tile_rows) {
+    const int ext_x = (P.N + 31) / 32 * 32;
+    const int ext_y = (P.N + tile_rows - 1) / tile_rows * tile_rows;
+    const int ext = ext_x > ext_y ? ext_x : ext_y;
+    const double R = fmax(P.half - 0.5, ext - 0.5 - P.half) * 1.4142135623730951;   // max |rho_c| of a tile pixel
+    const double f = 0.70710677, rz = (double)P.rhozero, dr = (double)P.deltarho;
+    const double margin = 1e-2 + 1e-5 * (R + fabs(rz)) / dr;
+    const double lo = ceil((-R - f - rz) / dr - margin), hi = ceil((R - f - rz) / dr + margin);
+    const int base = P.rpp > 2 ? 4 : 2;
+    const double need = fmax((double)base, fmax(-lo, hi - P.D + (double)base));
+    PairRows r;
+    r.inrange = need <= (double)kBpMaxPad;
+    r.pad = r.inrange ? (int)need : base;
+    r.W = P.D + 2 * r.pad - 1;
+    return r;
 }
 
 // The near-axis angles of list[0..nexact) for the PIX pixels, the reference's

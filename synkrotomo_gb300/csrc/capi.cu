@@ -244,16 +244,18 @@ int backward(synk_context *ctx, float *out, const float *angles, int64_t a, floa
     cudaStream_t st = ctx->stream;
     Scratch sc(st);
     AngleGeom *geom;
-    SYNK_CUDA(sc.reserve(Scratch::round(sizeof(AngleGeom) * (size_t)a) +
-                         Scratch::round(sizeof(float) * 2 * (size_t)p) + lists_bytes(a)),
+    float *pairs = nullptr;   // rows of detector pairs (launch_bp)
+    ProbGeom P = make_geom(a, rhozero, deltarho, numrhos, size_in, nullptr);
+    const size_t npair = bp_uses_pairs(P) ? bp_pairs_floats(P) : 0;
+    SYNK_CUDA(sc.reserve(Scratch::round(sizeof(AngleGeom) * (size_t)a) + Scratch::round(sizeof(float) * npair) +
+                         lists_bytes(a)),
               "cudaMallocAsync(scratch)");
     SYNK_CUDA(sc.get(&geom, (size_t)a), "cudaMallocAsync(geometry)");
-    const ProbGeom P = make_geom(a, rhozero, deltarho, numrhos, size_in, geom);
+    P.geom = geom;
     AngleLists L;
     SYNK_CUDA(make_setup(sc, angles, P, &L, st), "setup kernel");
-    float *scaled;   // scaled rows, or scaled detector pairs (launch_bp)
-    SYNK_CUDA(sc.get(&scaled, 2 * (size_t)p), "cudaMallocAsync(scaled rows)");
-    SYNK_CUDA(launch_bp(P, L, projections, out, st, scaled), "backprojection kernel");
+    if (npair) SYNK_CUDA(sc.get(&pairs, npair), "cudaMallocAsync(detector pairs)");
+    SYNK_CUDA(launch_bp(P, L, projections, out, st, pairs), "backprojection kernel");
     return SYNK_OK;
 }
 

@@ -10,12 +10,15 @@
 //                              one detector x 32 angles per warp)
 //             fp_det_kernel    fewer than kFpDetAngles angles: one warp = 32 detectors of one angle
 //             fp_exact_kernel  near-axis angles, the reference's expressions
-//   backward: bp_tile_kernel   one block = 32 x 8*PIX pixels, PIX = 4 or 8 per thread, all angles
-//             bp_split_kernel  the same with the angles split over warps (images too small
-//                              for one block per tile to fill the GPU)
+//   backward: row_pair_kernel  the sinogram's rows as scaled detector pairs
+//             bp_tile_kernel   one block = 32 columns, 4 or 8 pixels per thread, the angles split
+//                              over warps where the tiles would not fill the GPU
+//             bp_rows_kernel   the same from the plain rows (no scratch, more than four candidates)
 // See fp_tile.cuh and bp_tile.cuh for the per-ray and per-pixel arithmetic.
 #include <limits.h>
 #include <math.h>
+
+#include <type_traits>
 
 #include "synk_internal.cuh"
 #include "fp_tile.cuh"
@@ -526,180 +529,213 @@ cudaError_t launch_fp(const ProbGeom &P, const AngleLists &L, const float2 *xpai
 
 // ---- backprojection ---------------------------------------------------------------
 
-// sino_s[k][r] = sino[k][r] * row_scale(k): the rows of a SCALED backprojection.
-__global__ void __launch_bounds__(256) row_scale_kernel(ProbGeom P, const float *__restrict__ sino,
-                                                        float *__restrict__ sino_s) {
-    const int r = blockIdx.x * 256 + threadIdx.x;
-    const int k = blockIdx.y;
-    if (r >= P.D) return;
-    const size_t i = (size_t)k * P.D + r;
-    sino_s[i] = sino[i] * row_scale(P.geom, k);
-}
-
-// pair[k][s] = (v[s], v[s+1]) with v = sino[k] * row_scale(k) and v[D] = 0:
-// the rows of a SCALED backprojection as detector pairs (bp_chunk_pair).
-__global__ void __launch_bounds__(256) row_pair_kernel(ProbGeom P, const float *__restrict__ sino,
+// The rows of bp_chunk_pair: entry j of row k is (v[s], v[s+1]), s = j - pad, with
+// v = sino[k] * row_scale(k), zero outside [0, D) and for an angle without a direction.
+__global__ void __launch_bounds__(256) row_pair_kernel(ProbGeom P, int W, int pad, const float *__restrict__ sino,
                                                        float2 *__restrict__ pair) {
-    const int r = blockIdx.x * 256 + threadIdx.x;
-    const int k = blockIdx.y;
-    if (r >= P.D) return;
-    const size_t i = (size_t)k * P.D + r;
-    const float sc = row_scale(P.geom, k);
-    const float v1 = r + 1 < P.D ? sino[i + 1] * sc : 0.0f;
-    pair[i] = make_float2(sino[i] * sc, v1);
+    const int j = blockIdx.x * 256 + threadIdx.x;
+    if (j >= W) return;
+    const int s = j - pad;
+    for (int k = blockIdx.y; k < P.a; k += gridDim.y) {
+        float2 v = make_float2(0.0f, 0.0f);
+        if (isfinite(__ldg(&P.geom[k].c))) {
+            const float sc = row_scale(P.geom, k);
+            const float *row = sino + (size_t)k * P.D;
+            if ((unsigned)s < (unsigned)P.D) v.x = row[s] * sc;
+            if ((unsigned)(s + 1) < (unsigned)P.D) v.y = row[s + 1] * sc;
+        }
+        pair[(size_t)k * W + j] = v;
+    }
 }
 
-// Pixels per thread of the standalone backprojector (rows 8 apart: a block
-// covers 32 columns x 8*PIX rows), and the resident blocks per SM each variant
-// is compiled for.  8 pixels halve the per-angle overhead (dense data: 4.80 ms
-// against 5.02 at N = 2048, 2048 angles); 4 give twice the blocks, which the
-// few-angle (sparse-view) calls need.
-template <int PIX>
-struct BpShape {
-    static constexpr int kMinBlocks = PIX == 8 ? 5 : 6;
-};
-constexpr int kBpManyAngles = 256;     // angle count from which the 8-pixel variant runs
+// Pixels per thread of the standalone backprojector: 8 halve the per-angle
+// overhead (dense data: 4.80 ms against 5.02 at N = 2048, 2048 angles); 4 give
+// twice the blocks, which the few-angle (sparse-view) calls need.
+constexpr int kBpManyAngles = 256;     // angle count from which the 8-pixel variants run
 
-// sino_s: the fast-path rows (scaled when SCALED, else sino itself); sino:
-// the unscaled rows read by the near-axis angles.
-// PAIR (the dense in-range path): bp_chunk_pair.
-template <int kBpPix, bool UNIT, bool INRANGE, bool SCALED, bool PAIR = false>
-__global__ void __launch_bounds__(256, PAIR ? 3 : BpShape<kBpPix>::kMinBlocks) bp_tile_kernel(ProbGeom P, AngleLists L,
-                                                                   const float *__restrict__ sino_s,
-                                                                   const float *__restrict__ sino,
-                                                                   float *__restrict__ out) {
+// One block = 8/SB warp rows x SB angle parts, 32 x (8/SB)*PIX pixels, PIX rows
+// 8/SB apart per thread; SB = 1, 2, 4, 8 for images whose tiles are too few to
+// fill the GPU.  The SB partial sums of a pixel are added in a fixed order
+// through shared memory.  A warp's lanes are 8 columns x 4 rows where the block
+// has four rows (else 16 x 2, 32 x 1), so one angle's gathers of a warp span
+// fewer detectors than 32 columns of one row (4.15 -> 4.09 ms at N=2048, 2048
+// angles; 16 x 2: 4.11).  The FMA pipe and the issue slots bound it (9-10 warp
+// instructions per pixel and angle at deltarho 1); before, only whole angle sets
+// of in-range tiles read pairs, all else took two predicated scalar gathers per
+// pixel and angle.  us per call from the plain rows / from pairs: N=1000, 700 angles 651 /
+// 439; N=2046, 1999 angles 6419 / 3372; N=1500, 100 angles 217 / 135; N=512, 60
+// angles 36.8 / 30.6; deltarho 0.5, N=2048, 2048 angles 18900 / 6221 and N=362, 271
+// angles 139 / 82; deltarho 1.5, N=1000, 700 angles 1374 / 402; a detector row 300
+// short (clamped), N=512, 360 angles 108 / 90.
+template <int PIX, int RPP, bool UNIT, bool CLAMP, bool SPLIT>
+__global__ void __launch_bounds__(256, PIX == 8 ? 3 : 4) bp_tile_kernel(ProbGeom P, AngleLists L, int W, int pad,
+                                                                        const float2 *__restrict__ pairs,
+                                                                        const float *__restrict__ sino,
+                                                                        float *__restrict__ out, int lg) {
     __shared__ BpStage st;
+    __shared__ float red[SPLIT ? 8 : 1][PIX][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // PAIR: a warp's lanes are 8 columns x 4 rows of the tile (rows 8 apart per
-    // pixel m as before), so one angle's gathers of a warp span fewer
-    // detectors than 32 columns of one row (4.15 -> 4.09 ms; 16 x 2: 4.11)
-    const int col = PAIR ? blockIdx.x * 32 + (warp & 3) * 8 + (lane & 7) : blockIdx.x * 32 + lane;
-    const int row0 = PAIR ? blockIdx.y * (8 * kBpPix) + (warp >> 2) * 4 + (lane >> 3)
-                          : blockIdx.y * (8 * kBpPix) + warp;
+    const int lgSB = SPLIT ? lg : 0, SB = 1 << lgSB, RB = 8 >> lgSB;
+    const int part = warp & (SB - 1), wrow = warp >> lgSB;
+    const int lgR = RB >= 4 ? 2 : RB >> 1, lgC = 5 - lgR;      // a warp's rows and columns (log2)
+    const int col = blockIdx.x * 32 + ((wrow & ((1 << lgR) - 1)) << lgC) + (lane & ((1 << lgC) - 1));
+    const int row0 = blockIdx.y * (RB * PIX) + ((wrow >> lgR) << lgR) + (lane >> lgC);
     const float xc = (float)(col - P.half) + 0.5f;
     const float yc0 = (float)(row0 - P.half) + 0.5f;
-    float sum[kBpPix], comp[kBpPix];
+    float sum[PIX], comp[PIX];
 #pragma unroll
-    for (int m = 0; m < kBpPix; ++m) sum[m] = comp[m] = 0.0f;
+    for (int m = 0; m < PIX; ++m) sum[m] = comp[m] = 0.0f;
     for (int kc = 0; kc < P.a; kc += kBpChunk) {
         __syncthreads();
         bp_stage(P, kc, st);
         __syncthreads();
-        float part[kBpPix];
+        float prt[PIX];
+        bp_chunk_pair<PIX, RPP, UNIT, CLAMP>(P, st, kc, pairs, W, pad, part, lgSB, xc, yc0, (float)RB, prt);
 #pragma unroll
-        for (int m = 0; m < kBpPix; ++m) part[m] = 0.0f;
-        if constexpr (PAIR)
-            bp_chunk_pair<kBpPix>(P, st, kc, reinterpret_cast<const float2 *>(sino_s), xc, yc0, 8.0f, part);
-        else bp_chunk<kBpPix, UNIT, INRANGE, SCALED, 2>(P, st, kc, P.a, 0, 1, sino_s, xc, yc0, 8.0f, part);
-#pragma unroll
-        for (int m = 0; m < kBpPix; ++m) comp_add(sum[m], comp[m], part[m]);
+        for (int m = 0; m < PIX; ++m) comp_add(sum[m], comp[m], prt[m]);
     }
-    float ex[kBpPix];
+    float ex[PIX];
 #pragma unroll
-    for (int m = 0; m < kBpPix; ++m) ex[m] = 0.0f;
-    bp_exact_angles<kBpPix>(P, L.exact, __ldg(L.counts + 2), 0, 1, sino, row0, 8, col, ex);
+    for (int m = 0; m < PIX; ++m) ex[m] = 0.0f;
+    bp_exact_angles<PIX>(P, L.exact, __ldg(L.counts + 2), part, SB, sino, row0, RB, col, ex);
 #pragma unroll
-    for (int m = 0; m < kBpPix; ++m) {
-        const int row = row0 + 8 * m;
-        if (row < P.N && col < P.N) out[(size_t)row * P.N + col] = (sum[m] + comp[m]) + ex[m];
-    }
-}
-
-// The same pixels with the angles split SB ways (SB = 2, 4, 8), for images
-// whose 32 x 8*PIX tiles are too few to fill the GPU: a block = 8/SB warp
-// rows x SB angle parts, 32 x (8/SB)*PIX pixels; the SB partial sums of a
-// pixel are added in a fixed order through shared memory.
-template <int kBpPix, bool UNIT, bool INRANGE, bool SCALED>
-__global__ void __launch_bounds__(256, BpShape<kBpPix>::kMinBlocks) bp_split_kernel(ProbGeom P, AngleLists L,
-                                                                    const float *__restrict__ sino_s,
-                                                                    const float *__restrict__ sino,
-                                                                    float *__restrict__ out, int SB) {
-    __shared__ BpStage st;
-    __shared__ float red[8][kBpPix][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int RB = 8 / SB;
-    const int part = warp % SB, wrow = warp / SB;
-    const int col = blockIdx.x * 32 + lane;
-    const int row0 = blockIdx.y * (RB * kBpPix) + wrow;
-    const float xc = (float)(col - P.half) + 0.5f;
-    const float yc0 = (float)(row0 - P.half) + 0.5f;
-    float sum[kBpPix], comp[kBpPix];
+    for (int m = 0; m < PIX; ++m) ex[m] += sum[m] + comp[m];
+    if constexpr (SPLIT) {
 #pragma unroll
-    for (int m = 0; m < kBpPix; ++m) sum[m] = comp[m] = 0.0f;
-    for (int kc = 0; kc < P.a; kc += kBpChunk) {
+        for (int m = 0; m < PIX; ++m) red[warp][m][lane] = ex[m];
         __syncthreads();
-        bp_stage(P, kc, st);
-        __syncthreads();
-        float prt[kBpPix];
+        if (part != 0) return;
+        for (int t = 1; t < SB; ++t)
 #pragma unroll
-        for (int m = 0; m < kBpPix; ++m) prt[m] = 0.0f;
-        bp_chunk<kBpPix, UNIT, INRANGE, SCALED, 2>(P, st, kc, P.a, part, SB, sino_s, xc, yc0, (float)RB, prt);
-#pragma unroll
-        for (int m = 0; m < kBpPix; ++m) comp_add(sum[m], comp[m], prt[m]);
+            for (int m = 0; m < PIX; ++m) ex[m] += red[warp + t][m][lane];
     }
-    float ex[kBpPix];
 #pragma unroll
-    for (int m = 0; m < kBpPix; ++m) ex[m] = 0.0f;
-    bp_exact_angles<kBpPix>(P, L.exact, __ldg(L.counts + 2), part, SB, sino, row0, RB, col, ex);
-#pragma unroll
-    for (int m = 0; m < kBpPix; ++m) red[warp][m][lane] = (sum[m] + comp[m]) + ex[m];
-    __syncthreads();
-    if (part != 0) return;
-#pragma unroll
-    for (int m = 0; m < kBpPix; ++m) {
-        float v = red[warp][m][lane];
-        for (int t = 1; t < SB; ++t) v += red[warp + t][m][lane];
+    for (int m = 0; m < PIX; ++m) {
         const int row = row0 + RB * m;
-        if (row < P.N && col < P.N) out[(size_t)row * P.N + col] = v;
+        if (row < P.N && col < P.N) out[(size_t)row * P.N + col] = ex[m];
     }
 }
 
-// Angle split of the backprojection: the smallest SB whose tiles give at
+// Unscaled rows, any deltarho and row length: calls that have no memory for pairs
+// (noalloc), more than four candidates per pixel, and rows so long that a chunk
+// of pairs passes 4 GB.  A warp = 32 columns of one row.
+template <int PIX, bool UNIT, bool INRANGE>
+__global__ void __launch_bounds__(256, PIX == 8 ? 4 : 5) bp_rows_kernel(ProbGeom P, AngleLists L,
+                                                                        const float *__restrict__ sino,
+                                                                        float *__restrict__ out, int lgSB) {
+    __shared__ BpStage st;
+    __shared__ float red[8][PIX][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int SB = 1 << lgSB, RB = 8 >> lgSB;
+    const int part = warp & (SB - 1), wrow = warp >> lgSB;
+    const int col = blockIdx.x * 32 + lane;
+    const int row0 = blockIdx.y * (RB * PIX) + wrow;
+    const float xc = (float)(col - P.half) + 0.5f;
+    const float yc0 = (float)(row0 - P.half) + 0.5f;
+    float sum[PIX], comp[PIX];
+#pragma unroll
+    for (int m = 0; m < PIX; ++m) sum[m] = comp[m] = 0.0f;
+    for (int kc = 0; kc < P.a; kc += kBpChunk) {
+        __syncthreads();
+        bp_stage(P, kc, st);
+        __syncthreads();
+        float prt[PIX];
+#pragma unroll
+        for (int m = 0; m < PIX; ++m) prt[m] = 0.0f;
+        bp_chunk<PIX, UNIT, INRANGE, false, 2>(P, st, kc, P.a, part, SB, sino, xc, yc0, (float)RB, prt);
+#pragma unroll
+        for (int m = 0; m < PIX; ++m) comp_add(sum[m], comp[m], prt[m]);
+    }
+    float ex[PIX];
+#pragma unroll
+    for (int m = 0; m < PIX; ++m) ex[m] = 0.0f;
+    bp_exact_angles<PIX>(P, L.exact, __ldg(L.counts + 2), part, SB, sino, row0, RB, col, ex);
+#pragma unroll
+    for (int m = 0; m < PIX; ++m) ex[m] += sum[m] + comp[m];
+    if (SB > 1) {
+#pragma unroll
+        for (int m = 0; m < PIX; ++m) red[warp][m][lane] = ex[m];
+        __syncthreads();
+        if (part != 0) return;
+        for (int t = 1; t < SB; ++t)
+#pragma unroll
+            for (int m = 0; m < PIX; ++m) ex[m] += red[warp + t][m][lane];
+    }
+#pragma unroll
+    for (int m = 0; m < PIX; ++m) {
+        const int row = row0 + RB * m;
+        if (row < P.N && col < P.N) out[(size_t)row * P.N + col] = ex[m];
+    }
+}
+
+// Angle split of the backprojection (log2): the smallest SB whose tiles give at
 // least four blocks per SM (1 when the unsplit tiles already do), with at
 // least 8 angles per part (a split of a few angles only idles warps).
 static int bp_angle_split(const ProbGeom &P, int pix) {
     const long long want = 4LL * device_sms();
     const long long cols = (P.N + 31) / 32;
-    const int maxs = P.a >= 64 ? 8 : (P.a >= 32 ? 4 : (P.a >= 16 ? 2 : 1));
-    int SB = 1;
-    while (SB < maxs && cols * ((P.N + (8 / SB) * pix - 1) / ((8 / SB) * pix)) < want) SB *= 2;
-    return SB;
+    const int maxs = P.a >= 64 ? 3 : (P.a >= 32 ? 2 : (P.a >= 16 ? 1 : 0));
+    int lg = 0;
+    while (lg < maxs && cols * ((P.N + (8 >> lg) * pix - 1) / ((8 >> lg) * pix)) < want) ++lg;
+    return lg;
 }
 
-template <int PIX, bool SCALED>
-static void launch_bp_pix(const ProbGeom &P, const AngleLists &L, const float *sino_s, const float *sino, float *img,
-                          cudaStream_t stream) {
-    const int SB = bp_angle_split(P, PIX);
-    const bool inrange = bp_windows_in_range(P, 8 * PIX);    // split tiles (8/SB)*PIX rows high divide 8*PIX
-    const bool unit = P.deltarho == 1.0f;
-    if (SB == 1) {
-        const dim3 grid((P.N + 31) / 32, (P.N + 8 * PIX - 1) / (8 * PIX));
-        if (inrange) bp_tile_kernel<PIX, true, true, SCALED><<<grid, 256, 0, stream>>>(P, L, sino_s, sino, img);
-        else if (unit) bp_tile_kernel<PIX, true, false, SCALED><<<grid, 256, 0, stream>>>(P, L, sino_s, sino, img);
-        else bp_tile_kernel<PIX, false, false, SCALED><<<grid, 256, 0, stream>>>(P, L, sino_s, sino, img);
-    } else {
-        const int th = (8 / SB) * PIX;
-        const dim3 grid((P.N + 31) / 32, (P.N + th - 1) / th);
-        if (inrange) bp_split_kernel<PIX, true, true, SCALED><<<grid, 256, 0, stream>>>(P, L, sino_s, sino, img, SB);
-        else if (unit) bp_split_kernel<PIX, true, false, SCALED><<<grid, 256, 0, stream>>>(P, L, sino_s, sino, img, SB);
-        else bp_split_kernel<PIX, false, false, SCALED><<<grid, 256, 0, stream>>>(P, L, sino_s, sino, img, SB);
-    }
+template <int PIX>
+static void launch_bp_rows(const ProbGeom &P, const AngleLists &L, const float *sino, float *img,
+                           cudaStream_t stream) {
+    const int lg = bp_angle_split(P, PIX), th = (8 >> lg) * PIX;
+    const dim3 grid((P.N + 31) / 32, (P.N + th - 1) / th);
+    if (bp_windows_in_range(P, 8 * PIX)) bp_rows_kernel<PIX, true, true><<<grid, 256, 0, stream>>>(P, L, sino, img, lg);
+    else if (P.deltarho == 1.0f) bp_rows_kernel<PIX, true, false><<<grid, 256, 0, stream>>>(P, L, sino, img, lg);
+    else bp_rows_kernel<PIX, false, false><<<grid, 256, 0, stream>>>(P, L, sino, img, lg);
 }
+
+template <int PIX>
+static void launch_bp_pairs(const ProbGeom &P, const AngleLists &L, const float *sino, float2 *pairs, float *img,
+                            cudaStream_t stream) {
+    const PairRows R = bp_pair_rows(P, 8 * PIX);      // split tiles (8/SB)*PIX rows high divide 8*PIX
+    row_pair_kernel<<<dim3((R.W + 255) / 256, P.a < 65535 ? P.a : 65535), 256, 0, stream>>>(P, R.W, R.pad, sino, pairs);
+    const int lg = bp_angle_split(P, PIX), th = (8 >> lg) * PIX;
+    const dim3 grid((P.N + 31) / 32, (P.N + th - 1) / th);
+    auto run = [&](auto rpp, auto unit, auto clamp) {
+        constexpr int RPP = decltype(rpp)::value;
+        constexpr bool UNIT = decltype(unit)::value, CLAMP = decltype(clamp)::value;
+        if (lg) bp_tile_kernel<PIX, RPP, UNIT, CLAMP, true><<<grid, 256, 0, stream>>>(P, L, R.W, R.pad, pairs, sino, img, lg);
+        else bp_tile_kernel<PIX, RPP, UNIT, CLAMP, false><<<grid, 256, 0, stream>>>(P, L, R.W, R.pad, pairs, sino, img, 0);
+    };
+    auto range = [&](auto rpp, auto unit) {
+        if (R.inrange) run(rpp, unit, std::false_type());
+        else run(rpp, unit, std::true_type());
+    };
+    if (P.deltarho == 1.0f) range(std::integral_constant<int, 2>(), std::true_type());
+    else if (P.rpp == 1) range(std::integral_constant<int, 1>(), std::false_type());
+    else if (P.rpp == 2) range(std::integral_constant<int, 2>(), std::false_type());
+    else if (P.rpp == 3) range(std::integral_constant<int, 3>(), std::false_type());
+    else range(std::integral_constant<int, 4>(), std::false_type());
+}
+
+// Rows of pairs in the launch of P (tiles of 8 or 4 pixels per thread).
+static PairRows launch_pair_rows(const ProbGeom &P) { return bp_pair_rows(P, P.a >= kBpManyAngles ? 64 : 32); }
+
+// Pairs for up to four candidates (deltarho >= 0.354): more would need variants of
+// their own.  A chunk's rows must stay within the 32-bit gather offsets.
+bool bp_uses_pairs(const ProbGeom &P) {
+    return P.rpp <= 4 &&
+           (unsigned long long)(P.a < kBpChunk ? P.a : kBpChunk) * launch_pair_rows(P).W * 8ull < (1ull << 32);
+}
+
+size_t bp_pairs_floats(const ProbGeom &P) { return 2 * (size_t)P.a * (size_t)launch_pair_rows(P).W; }
 
 cudaError_t launch_bp(const ProbGeom &P, const AngleLists &L, const float *sino, float *img, cudaStream_t stream,
-                      float *scaled) {
-    if (scaled && P.a >= kBpManyAngles && bp_angle_split(P, 8) == 1 && bp_windows_in_range(P, 64)) {
-        // dense data: detector pairs, one 8-byte gather per (pixel, angle)
-        row_pair_kernel<<<dim3((P.D + 255) / 256, P.a), 256, 0, stream>>>(P, sino, reinterpret_cast<float2 *>(scaled));
-        const dim3 grid((P.N + 31) / 32, (P.N + 63) / 64);
-        bp_tile_kernel<8, true, true, true, true><<<grid, 256, 0, stream>>>(P, L, scaled, sino, img);
-    } else if (scaled) {
-        row_scale_kernel<<<dim3((P.D + 255) / 256, P.a), 256, 0, stream>>>(P, sino, scaled);
-        if (P.a >= kBpManyAngles) launch_bp_pix<8, true>(P, L, scaled, sino, img, stream);
-        else launch_bp_pix<4, true>(P, L, scaled, sino, img, stream);
+                      float *pairs) {
+    const bool many = P.a >= kBpManyAngles;
+    if (pairs) {
+        float2 *p2 = reinterpret_cast<float2 *>(pairs);
+        if (many) launch_bp_pairs<8>(P, L, sino, p2, img, stream);
+        else launch_bp_pairs<4>(P, L, sino, p2, img, stream);
     } else {
-        if (P.a >= kBpManyAngles) launch_bp_pix<8, false>(P, L, sino, sino, img, stream);
-        else launch_bp_pix<4, false>(P, L, sino, sino, img, stream);
+        if (many) launch_bp_rows<8>(P, L, sino, img, stream);
+        else launch_bp_rows<4>(P, L, sino, img, stream);
     }
     return cudaGetLastError();
 }

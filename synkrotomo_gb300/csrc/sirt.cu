@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(256, MINB) sirt_bp_stack_kernel(SirtProblem q,
         bp_stage(P, kc, st);
         __syncthreads();
         float part[8];
-        bp_chunk_pair<8>(P, st, kc, rows, xc, yc0, 8.0f, part);
+        bp_chunk_pair<8>(P, st, kc, rows, P.D, 0, 0, 0, xc, yc0, 8.0f, part);
 #pragma unroll
         for (int m = 0; m < 8; ++m) comp_add(sum[m], comp[m], part[m]);
     }

@@ -395,11 +395,12 @@ int device_sms();
 cudaError_t launch_geometry(const float *angles, int a, AngleGeom *geom, cudaStream_t stream);
 cudaError_t launch_fp(const ProbGeom &P, const AngleLists &L, const float2 *xpair, const float2 *xTpair, float *sino,
                       cudaStream_t stream);
-// scaled: scratch of 2*a*D floats for the lbase-scaled rows (faster inner
-// loop; detector pairs on the dense in-range path), or null for the unscaled
-// kernel (no scratch)
+// pairs: scratch of bp_pairs_floats(P) floats for the rows of scaled detector
+// pairs (where bp_uses_pairs(P)), or null for the kernel without scratch
+bool bp_uses_pairs(const ProbGeom &P);
+size_t bp_pairs_floats(const ProbGeom &P);
 cudaError_t launch_bp(const ProbGeom &P, const AngleLists &L, const float *sino, float *img, cudaStream_t stream,
-                      float *scaled);
+                      float *pairs);
 // R, C and the lists of rays that only clip a corner pixel (their R stored
 // negated; graze [4*capc] entries {k, r} by corner in ray order, glen
 // [4*capc] their chords, goff [5] the prefix offsets; graze_tmp / glen_tmp
