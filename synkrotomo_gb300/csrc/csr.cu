@@ -34,7 +34,7 @@ __device__ __forceinline__ float ray_intercept(const ProbGeom &P, const AngleGeo
     return __fdiv_rn(rho, g.cost);
 }
 
-// The forward rule at one frame row, fast path (see fp_rows_fast).
+// The forward rule at one frame row, fast path (see ones_rows).
 __device__ __forceinline__ RowEntries row_fast(const ProbGeom &P, const AngleGeom &g, float u0, int j) {
     RowEntries e;
     const float u = fmaf((float)j, g.slope, u0);
@@ -75,7 +75,7 @@ __device__ __forceinline__ bool ray_in_range(const ProbGeom &P, float rho) {
     return !(fabsf(rho) > 0.75f * (float)P.N + 2.0f);
 }
 
-// Frame row range of a fast-path ray (as fp_ray clips it).
+// Frame row range of a fast-path ray (as ray_rows clips it).
 __device__ __forceinline__ void fast_rows(const ProbGeom &P, const AngleGeom &g, float u0, int &j0, int &j1) {
     j0 = 0;
     j1 = P.N;

@@ -764,19 +764,45 @@ __device__ __forceinline__ int graze_corner(const AngleGeom &g, float rho) {
 // orders them) and its R is stored negated, which sends it to the SIRT
 // kernels' exact treatment (sirt.cu).  A ray without a slot (not reached with
 // the caller's bound) keeps the fast path.
+//
+// In the rows in which both of a ray's pixels lie inside the image their shares
+// add up to exactly 1, so only the rows at its ends are evaluated and the others
+// counted; a near-axis angle's rows are split over the block's warps.  What is
+// left is latency (figures at colnorm_kernel).
 __global__ void __launch_bounds__(256) rownorm_kernel(ProbGeom P, float *__restrict__ R, int2 *__restrict__ graze,
                                                       float *__restrict__ glen, int *__restrict__ gcnt, int capc) {
+    __shared__ double red[8][32];
+    __shared__ int near[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k = blockIdx.y * 8 + warp;
     const int r = blockIdx.x * 32 + lane;
+    const float rho = __fadd_rn(P.rhozero, __fmul_rn((float)r, P.deltarho));
+    const bool reach = !(fabsf(rho) > 0.75f * (float)P.N + 2.0f);
+    const AngleGeom g = load_geom(P.geom, min(k, P.a - 1));
+    if (lane == 0) near[warp] = k < P.a && g.exact;
+    __syncthreads();
+    double v = 0.0;
+    if (k < P.a && !g.exact && reach) v = fp_ray_ones(P, g, rho);
+    for (int w = 0; w < 8; ++w) {
+        if (!near[w]) continue;                                  // block-uniform
+        const AngleGeom h = load_geom(P.geom, blockIdx.y * 8 + w);
+        const float intercept = __fdiv_rn(rho, h.cost);
+        double acc = 0.0;
+        if (reach)
+            for (int i = -P.half + P.N * warp / 8; i < -P.half + P.N * (warp + 1) / 8; ++i)
+                acc += (double)fp_row_exact<true>(nullptr, P.N, P.half, h.slope, intercept, h.lbase, i);
+        red[warp][lane] = acc;
+        __syncthreads();
+        if (warp == w)
+            for (int t = 0; t < 8; ++t) v += red[t][lane];
+        __syncthreads();
+    }
     if (k >= P.a || r >= P.D) return;
-    const AngleGeom g = load_geom(P.geom, k);
-    const double v = fp_ray<true>(P, g, nullptr, r, 0, P.N);
     float Rv = v != 0.0 ? (float)(1.0 / v) : 0.0f;
     if (v > 0.0 && v < 1.0 && !g.exact) {
         const float e = fp_ray_exact_f32<true>(P, g, nullptr, 0, r);
         if (e != 0.0f) {
-            const int c = graze_corner(g, __fadd_rn(P.rhozero, __fmul_rn((float)r, P.deltarho)));
+            const int c = graze_corner(g, rho);
             const int slot = atomicAdd(gcnt + c, 1);
             if (slot < capc) {
                 graze[(size_t)c * capc + slot] = make_int2(k, r);
@@ -830,19 +856,47 @@ __global__ void __launch_bounds__(1024) graze_sort_kernel(const int2 *__restrict
     }
 }
 
-// C = safe_inverse(A^T*1): one thread per pixel, FP64 angle sum (SIRT.fut:25).
+// C = safe_inverse(A^T*1), float32 sums over 32 angles, added in FP64
+// (SIRT.fut:25).  A block is 32 columns x 4 rows: each warp takes every eighth
+// group of 32 angles for all 128 pixels (four per lane, so an angle's constants
+// and branches serve four independent sums), then the warps' sums are added in
+// order.  RPP: candidates per pixel, 0 = any.  Bound by the issue slots.
+// Eight problems of N=128-512 and 60-360 angles together: 545 us with one thread
+// per pixel and all angles, 342 with the split, 269 with one branch for the four
+// pixels; rownorm_kernel 337 us with whole rays, 115 now.
+template <int RPP>
 __global__ void __launch_bounds__(256) colnorm_kernel(ProbGeom P, float *__restrict__ C) {
-    const int col = blockIdx.x * 32 + (threadIdx.x & 31);
-    const int row = blockIdx.y * 8 + (threadIdx.x >> 5);
-    if (row >= P.N || col >= P.N) return;
-    double dsum = 0.0;
-    for (int k0 = 0; k0 < P.a; k0 += 32) {
+    __shared__ double red[8][4][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int col = blockIdx.x * 32 + lane, row0 = blockIdx.y * 4;
+    if (RPP) P.rpp = RPP;
+    double dsum[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int k0 = warp * 32; k0 < P.a; k0 += 256) {
         const int k1 = min(k0 + 32, P.a);
-        float part = 0.0f;
-        for (int k = k0; k < k1; ++k) part += bp_angle<true>(P, load_geom(P.geom, k), nullptr, row, col);
-        dsum += (double)part;
+        float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int k = k0; k < k1; ++k) {
+            AngleGeom g = load_geom(P.geom, k);
+            const bool near = g.exact;                           // warp-uniform, one branch for the four pixels
+            g.exact = 0;
+            if (!near) {
+#pragma unroll
+                for (int m = 0; m < 4; ++m) part[m] += bp_angle<true>(P, g, nullptr, row0 + m, col);
+            } else {
+                g.exact = 1;
+                for (int m = 0; m < 4; ++m) part[m] += bp_angle<true>(P, g, nullptr, row0 + m, col);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) dsum[m] += (double)part[m];
     }
-    C[(size_t)row * P.N + col] = dsum != 0.0 ? (float)(1.0 / dsum) : 0.0f;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) red[warp][m][lane] = dsum[m];
+    __syncthreads();
+    const int row = row0 + warp;
+    if (warp >= 4 || row >= P.N || col >= P.N) return;
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += red[w][warp][lane];
+    C[(size_t)row * P.N + col] = t != 0.0 ? (float)(1.0 / t) : 0.0f;
 }
 
 cudaError_t launch_normalisers(const ProbGeom &P, float *R, float *C, int2 *graze, float *glen, int *goff,
@@ -856,8 +910,9 @@ cudaError_t launch_normalisers(const ProbGeom &P, float *R, float *C, int2 *graz
     graze_sort_kernel<<<1, 1024, 0, stream>>>(graze_tmp, glen_tmp, gcnt, graze, glen, goff, capc);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    dim3 gb((P.N + 31) / 32, (P.N + 7) / 8);
-    colnorm_kernel<<<gb, 256, 0, stream>>>(P, C);
+    dim3 gb((P.N + 31) / 32, (P.N + 3) / 4);
+    if (P.rpp == 2) colnorm_kernel<2><<<gb, 256, 0, stream>>>(P, C);
+    else colnorm_kernel<0><<<gb, 256, 0, stream>>>(P, C);
     return cudaGetLastError();
 }
 

@@ -133,50 +133,30 @@ __device__ __forceinline__ float right_share(float u, float fl, float ainv) {
     return __saturatef(__fmaf_rn(__fsub_rn(u, fl), ainv, __fsub_rn(1.0f, ainv)));
 }
 
-// ---------------------------------------------------------------------------
-// Forward projection of one ray: sum over the rows of the traversal frame.
-// img points at the image seen in that frame (the transposed image for flat
-// lines).  ONES replaces every in-bounds pixel by 1 (normaliser R, FP64 sum).
-// ---------------------------------------------------------------------------
-template <bool ONES>
-struct FpAcc;
-template <> struct FpAcc<false> { typedef float T; };
-template <> struct FpAcc<true> { typedef double T; };
-
-// Rows [j0, j1) of the fast path, accumulated into (sum, comp): partial sums
-// over 32 rows, compensated across partials.
-template <bool ONES>
-__device__ __forceinline__ void fp_rows_fast(const float *__restrict__ img, int N, float slope, float x0,
-                                             float ainv, int j0, int j1,
-                                             typename FpAcc<ONES>::T &sum, float &comp) {
+// Rows [j0, j1) of a fast-path ray over an image of ones: float32 sums of 32
+// rows, added in FP64.
+__device__ __forceinline__ double ones_rows(int N, float slope, float x0, float ainv, int j0, int j1) {
     const unsigned uN = (unsigned)N;
     const int half = N / 2;
+    double sum = 0.0;
     int j = j0;
     while (j < j1) {
         const int jend = min(j + 32, j1);
         float part = 0.0f;
-        const float *row = img + (size_t)j * N;
 #pragma unroll 4
-        for (; j < jend; ++j, row += N) {
+        for (; j < jend; ++j) {
             // x = left end of the row segment, centred; c = its pixel index
             const float x = fmaf((float)(j - half), slope, x0);
             int c;
             const float fl = floor_magic(x, c);
             c += half;
             const float t = right_share(x, fl, ainv);                      // share of pixel c+1
-            float v0, v1;
-            if constexpr (ONES) {
-                v0 = ((unsigned)c < uN) ? 1.0f : 0.0f;
-                v1 = ((unsigned)(c + 1) < uN) ? 1.0f : 0.0f;
-            } else {
-                v0 = ((unsigned)c < uN) ? __ldg(row + c) : 0.0f;
-                v1 = ((unsigned)(c + 1) < uN) ? __ldg(row + c + 1) : 0.0f;
-            }
+            const float v0 = ((unsigned)c < uN) ? 1.0f : 0.0f, v1 = ((unsigned)(c + 1) < uN) ? 1.0f : 0.0f;
             part += fmaf(t, v1 - v0, v0);
         }
-        if constexpr (ONES) sum += (double)part;
-        else comp_add(sum, comp, part);
+        sum += (double)part;
     }
+    return sum;
 }
 
 // One frame row of the reference's own expressions (forwardprojection.fut:
@@ -242,47 +222,29 @@ __device__ __forceinline__ ExactRow fp_row_exact_terms(int half, float slope, fl
     return e;
 }
 
-// All rows of a near-axis line, in the reference's order.
-template <bool ONES>
-__device__ __forceinline__ void fp_rows_exact(const float *__restrict__ img, int stride, int half, float slope,
-                                              float intercept, float lbase,
-                                              typename FpAcc<ONES>::T &sum) {
-    typename FpAcc<ONES>::T acc = 0;
-    for (int i = -half; i < half; ++i)
-        acc += (typename FpAcc<ONES>::T)fp_row_exact<ONES>(img, stride, half, slope, intercept, lbase, i);
-    sum = acc;
-}
-
-// Ray sum of detector r of the angle with geometry g.  Returns the reference
-// value sum_rows(lbot*img[bot] + ltop*img[top]) (lbase already applied).
-template <bool ONES>
-__device__ __forceinline__ typename FpAcc<ONES>::T fp_ray(const ProbGeom &P, const AngleGeom &g,
-                                                          const float *__restrict__ img_frame, int r,
-                                                          int jbeg, int jend) {
-    typedef typename FpAcc<ONES>::T T;
-    const float rho = __fadd_rn(P.rhozero, __fmul_rn((float)r, P.deltarho));   // forwardprojection.fut:28
-    const float intercept = __fdiv_rn(rho, g.cost);                               // forwardprojection.fut:29
-    // |rho| of any point of the image is at most N/sqrt(2): such a ray adds nothing
-    if (fabsf(rho) > 0.75f * (float)P.N + 2.0f) return (T)0;
-    if (g.exact) {
-        // whole ray in one piece (only the row-part starting at 0 computes it)
-        if (jbeg != 0) return (T)0;
-        T s;
-        fp_rows_exact<ONES>(img_frame, P.N, P.half, g.slope, intercept, g.lbase, s);   // unpadded frame
-        return s;
-    }
-    // x(j) = xlo(row j) centred, xlo = xbot + min(slope,0), xbot = (j-half)*slope + intercept
-    const float x0 = ray_x0(g, intercept);
+// Ray at distance rho over an image of ones (not a near-axis angle's).  Rows in which pixels c and
+// c+1 both lie inside the image add exactly 1; x is monotone in the row, also as
+// rounded, so two rows found inside prove the rows between them.
+__device__ __forceinline__ double fp_ray_ones(const ProbGeom &P, const AngleGeom &g, float rho) {
+    const float x0 = ray_x0(g, __fdiv_rn(rho, g.cost));
     int j0, j1;
     ray_rows(P, g, x0, j0, j1);
-    j0 = max(j0, jbeg);
-    j1 = min(j1, jend);
     if (j1 < j0) j1 = j0;
-    T sum = (T)0;
-    float comp = 0.0f;
-    fp_rows_fast<ONES>(img_frame, P.N, g.slope, x0, g.ainv, j0, j1, sum, comp);
-    if (ONES) return sum * (double)g.lbase;
-    return (T)(((float)sum + comp) * g.lbase);
+    const float inv = __fdiv_rn(1.0f, g.slope), h = (float)P.half;
+    const float ra = (0.25f - h - x0) * inv + h, rb = (h - 1.25f - x0) * inv + h;    // rows of the inner columns
+    const float lim = (float)P.N + 1.0f;                                              // NaN (no slope): all rows
+    int ja = max(j0, (int)fmaxf(fminf(fminf(ra, rb), lim), -1.0f) + 1);
+    int jb = min(j1, (int)fmaxf(fminf(fmaxf(ra, rb), lim), -1.0f));
+    auto inside = [&](int j) {
+        int c;
+        floor_magic(fmaf((float)(j - P.half), g.slope, x0), c);
+        c += P.half;
+        return c >= 0 && c + 1 < P.N;
+    };
+    if (!(jb > ja && inside(ja) && inside(jb - 1))) ja = jb = j1;
+    const double sum = ones_rows(P.N, g.slope, x0, g.ainv, j0, ja) + (double)(jb - ja) +
+                       ones_rows(P.N, g.slope, x0, g.ainv, jb, j1);
+    return sum * (double)g.lbase;
 }
 
 // ---------------------------------------------------------------------------
@@ -299,9 +261,9 @@ __device__ __forceinline__ float bp_angle(const ProbGeom &P, const AngleGeom &g,
         const float yc = (float)(row - half) + 0.5f;
         const float rhoc = fmaf(xc, g.c, -yc * g.s);
         int s0;
-        ceil_magic((rhoc - fact_f32() - P.rz_c) * P.inv_deltarho, s0);   // centred detector index
+        const float s0f = ceil_magic((rhoc - fact_f32() - P.rz_c) * P.inv_deltarho, s0);   // centred detector index
         float acc = 0.0f;
-        float d = fmaf((float)s0, P.deltarho, P.rz_c) - rhoc;
+        float d = fmaf(s0f, P.deltarho, P.rz_c) - rhoc;
         for (int q = 0; q < P.rpp; ++q, d += P.deltarho) {
             const int det = s0 + P.zi + q;
             const float w = __saturatef(fmaf(-fabsf(d), g.inv_b, g.h_over_b));
