@@ -30,6 +30,7 @@
 #include "synk_internal.cuh"
 #include "sirt_internal.cuh"
 #include "sirt_device.cuh"
+#include "sirt_offset.cuh"
 #include "fp_tile.cuh"
 #include "bp_tile.cuh"
 
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(1024, 1) sirt_small_kernel(const SirtSmall p) 
             h[o] = w ? g.h_over_b : -1.0f;
             ib[o] = w ? g.inv_b : 0.0f;
             c1[o] = w ? fmaf(-(1.0f - fact_f32()), g.inv_b, g.h_over_b) : -1.0f;
-            ro[o] = __uint_as_float(((unsigned)k * (unsigned)P.D + (unsigned)P.zi - (unsigned)kMagicBits) * 4u);
+            ro[o] = __uint_as_float(small_row_offset(k, P.D, P.zi, kMagicBits));
         }
         sh.cs[j] = make_float4(c[0], c[1], si[0], si[1]);
         sh.hb[j] = make_float4(h[0], h[1], ib[0], ib[1]);
@@ -424,7 +425,7 @@ __global__ void __launch_bounds__(1024, 1) sirt_small_kernel(const SirtSmall p) 
             }
             if (on) {
                 const float *rr = q.rr + (size_t)s * pr;
-                const char *rrb = reinterpret_cast<const char *>(rr);
+                const char *rrb = reinterpret_cast<const char *>(rr - kSmallLead);
                 const float xc = (float)(col - P.half) + 0.5f, yc = (float)(row - P.half) + 0.5f;
                 const f32x2 xc2 = pk2(xc, xc), nyc2 = pk2(-yc, -yc), zo2 = pk2(zoff, zoff);
                 const f32x2 mg2 = pk2(kMagic, kMagic), nmg2 = pk2(-kMagic, -kMagic), m1 = pk2(-1.0f, -1.0f);
@@ -446,8 +447,8 @@ __global__ void __launch_bounds__(1024, 1) sirt_small_kernel(const SirtSmall p) 
                         for (int o = 0; o < 2; ++o) {
                             const int i = 2 * h + o;
                             const float ib = o ? b4.w : b4.z;
-                            const unsigned off = (unsigned)__float_as_int(o ? rv.y : rv.x) * 4u +
-                                                 __float_as_uint(o ? c4.w : c4.z);
+                            const unsigned off = small_gather_offset(__float_as_uint(o ? rv.y : rv.x),
+                                                                     __float_as_uint(o ? c4.w : c4.z));
                             w0[i] = __saturatef(fmaf(-fabsf(o ? dv.y : dv.x), ib, o ? b4.y : b4.x));
                             w1[i] = __saturatef(fmaf(-(o ? ev.y : ev.x), ib, o ? c4.y : c4.x));
                             if (j0 + h >= jend) w0[i] = w1[i] = 0.0f;            // past the part's last pair
