@@ -133,6 +133,8 @@ __device__ __forceinline__ void fp_unit(const SirtProblem &q, SmallShared &sh, i
 // Sum of the unit's rows (fp_lane_walk's arithmetic, eight rows of gathers in
 // flight): v0 = pixel c, v1 = pixel c+1 of the padded frame image, the index
 // clamped to the zero entries N+1 and N+2 outside the image and past the last row.
+// A lane without a ray walks pixels that are not its own: its sum is dropped, not
+// multiplied by zero (the pixels may be infinite or NaN).
 __device__ __forceinline__ float small_walk(const ProbGeom &P, const float4 L, int J0, int J1, const float *img) {
     const unsigned W = (unsigned)(P.N + 2), zix = (unsigned)P.N + 1u;
     const unsigned okbase = (unsigned)kMagicBits - 1u - (unsigned)P.half;   // bits(r) - okbase = c + 1
@@ -174,7 +176,7 @@ __device__ __forceinline__ float small_walk(const ProbGeom &P, const float4 L, i
         }
     }
     comp_add(sum, comp, part);
-    return (sum + comp) * L.w;
+    return L.w != 0.0f ? (sum + comp) * L.w : 0.0f;
 }
 
 // Decodes extra x of the problem: slice by slice the near-axis rays, then the
