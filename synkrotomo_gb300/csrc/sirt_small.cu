@@ -268,10 +268,12 @@ __global__ void __launch_bounds__(1024, 1) sirt_small_kernel(const SirtSmall p) 
         for (int o = 0; o < 2; ++o) {
             const int k = min(2 * j + o, P.a - 1);
             const AngleGeom g = load_geom(P.geom, k);
-            // (no weight without a finite line, nor past the last angle)
-            const bool w = !g.exact && fabsf(g.c) <= 2.0f && 2 * j + o < P.a;
-            c[o] = w ? g.c : 0.0f;
-            si[o] = w ? g.s : 0.0f;
+            // no weight without a finite line, nor past the last angle, whose entries
+            // the filler of an odd count reads again: a detector outside a pixel's
+            // window must not enter it, not even times zero (it may be NaN)
+            const bool line = !g.exact && fabsf(g.c) <= 2.0f, w = line && 2 * j + o < P.a;
+            c[o] = line ? g.c : 0.0f;
+            si[o] = line ? g.s : 0.0f;
             h[o] = w ? g.h_over_b : -1.0f;
             ib[o] = w ? g.inv_b : 0.0f;
             c1[o] = w ? fmaf(-(1.0f - fact_f32()), g.inv_b, g.h_over_b) : -1.0f;

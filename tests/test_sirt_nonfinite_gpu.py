@@ -35,7 +35,8 @@ def _same(got, want):
     assert rel_l2(got[~bad], want[~bad]) < 1e-5
 
 
-@pytest.mark.parametrize("size,angles,row,col", [(64, 8, 20, 32), (130, 6, 100, 65), (66, 10, 3, 33)])
+@pytest.mark.parametrize("size,angles,row,col", [(64, 8, 20, 32), (130, 6, 100, 65), (66, 10, 3, 33),
+                                                 (64, 7, 20, 32)])
 def test_rays_that_miss_a_nan_pixel(gpu, size, angles, row, col):
     """The centre column is where lanes without a ray walk."""
     det = phantom.default_detectors(size)
@@ -44,3 +45,13 @@ def test_rays_that_miss_a_nan_pixel(gpu, size, angles, row, col):
     image = np.zeros((size, size), np.float32)
     image[row, col] = np.nan
     _same(_solve(ang, det, size, 1, image.ravel(), b, 0), _solve(ang, det, size, 1, image.ravel(), b, -1))
+
+
+@pytest.mark.parametrize("size,angles", [(64, 7), (130, 33), (66, 1)])
+def test_odd_angle_count_and_a_nan_detector(gpu, size, angles):
+    """The last angle of an odd count is read by the filler of its pair too."""
+    det = phantom.default_detectors(size)
+    ang = (0.31 + math.pi / angles * np.arange(angles)).astype(np.float32)
+    b = np.random.default_rng(size).random((angles, det)).astype(np.float32)
+    b[-1, det // 2] = np.nan
+    _same(_solve(ang, det, size, 1, None, b.ravel(), 0), _solve(ang, det, size, 1, None, b.ravel(), -1))
