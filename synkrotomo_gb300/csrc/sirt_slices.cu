@@ -335,7 +335,10 @@ __global__ void __launch_bounds__(256) sirt_fp_slices_exact_kernel(SirtProblem q
 //     lanes' entries lie within 8 of each other, so a shared one takes four.
 //   - Two pixels next to each other along the axis on which the detector
 //     coordinate moves less (|dq| <= sqrt(1/2)) share one window of three
-//     detectors: three gathers for two pixels instead of four.
+//     detectors: three gathers for two pixels instead of four.  The second pixel's
+//     own two are the first two or the last two, and the third gather is whichever
+//     of the outer ones it has: a detector outside a pixel's window must not enter
+//     it, not even times zero (it may be infinite or NaN).
 // Both together took 16 slices x 10 iterations at N=512 / 360 angles from 10.4
 // to 9.2 ms against unshared windows gathered from global memory.
 // The update x + C*bp and both padded copies are the epilogue.  More than
@@ -476,17 +479,21 @@ __global__ void __launch_bounds__(256, 4) sirt_bp_slices_kernel(SirtProblem q, i
                         const float wG1 = __saturatef(fmaf(-fabsf(o ? hGv.y : hGv.x), g.w, g.z));
                         const float wG2 = __saturatef(fmaf(-(o ? eGv.y : eGv.x), g.w, c2));
                         const unsigned ad = (unsigned)__float_as_int(o ? rv.y : rv.x) * EB + off;
-                        f32x2 v0[V / 2], v1[V / 2], v2[V / 2];
+                        const bool past = (o ? eGv.y : eGv.x) < 0.0f;
+                        f32x2 v0[V / 2], v1[V / 2], x[V / 2];
                         lds_pairs<V>(ad, v0);
                         lds_pairs<V>(ad + EB, v1);
-                        lds_pairs<V>(ad + 2 * EB, v2);
+                        lds_pairs<V>(past ? ad + 2 * EB : ad, x);
 #pragma unroll
                         for (int p = 0; p < V / 2; ++p) {
                             fa[p] = fma2(pk2(wF0, wF0), v0[p], fa[p]);
                             fa[p] = fma2(pk2(wF1, wF1), v1[p], fa[p]);
-                            ga[p] = fma2(pk2(wG0, wG0), v0[p], ga[p]);
+                        }
+                        const float wx = past ? wG2 : wG0;
+#pragma unroll
+                        for (int p = 0; p < V / 2; ++p) {
+                            ga[p] = fma2(pk2(wx, wx), x[p], ga[p]);
                             ga[p] = fma2(pk2(wG1, wG1), v1[p], ga[p]);
-                            ga[p] = fma2(pk2(wG2, wG2), v2[p], ga[p]);
                         }
                     }
                 };

@@ -55,3 +55,17 @@ def test_odd_angle_count_and_a_nan_detector(gpu, size, angles):
     b = np.random.default_rng(size).random((angles, det)).astype(np.float32)
     b[-1, det // 2] = np.nan
     _same(_solve(ang, det, size, 1, None, b.ravel(), 0), _solve(ang, det, size, 1, None, b.ravel(), -1))
+
+
+@pytest.mark.parametrize("size,angles,ns", [(256, 45, 12), (250, 45, 13), (160, 271, 6)])
+def test_stack_with_a_nan_detector(gpu, size, angles, ns):
+    """Neighbouring pixels of the interleaved slices share a window of three
+    detectors, of which a pixel's own are two."""
+    det = phantom.default_detectors(size)
+    assert ns * angles * size * (size + det) > 6.5e7
+    ang = (0.31 + math.pi / angles * np.arange(angles)).astype(np.float32)
+    b = np.random.default_rng(size).random((ns, angles, det)).astype(np.float32)
+    b[1, 3, det // 3] = np.nan
+    b[-1, 7, det // 2 + 11] = np.nan
+    _same(_solve(ang, det, size, ns, None, b.ravel(), 0),
+          _solve(ang, det, size, ns, None, b.ravel(), rt.resident_blocks()))
