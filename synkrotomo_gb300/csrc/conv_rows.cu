@@ -351,6 +351,7 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
             // one decision for the four warps (an accumulator is only ever signalled whole:
             // the error word needs no look here, a trip to L2 per row)
             if (!epi_and(bar, ok)) break;
+            __syncwarp();                              // the lanes leave the waits one by one, TMEM is read together
             tc_fence_after();
             uint8_t *tile = gio + (size_t)j * p.io_bytes;
             const uint32_t tbase = tmem + slot * (uint32_t)p.N + ((uint32_t)(q4 * 32) << 16);
@@ -405,6 +406,7 @@ __global__ void __launch_bounds__(320, 1) conv_rows_kernel(const __grid_constant
                     load_mask();
                 }
             }
+            __syncwarp();
             slot += 2;
             if (slot >= nb) {
                 slot -= nb;
