@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(192, 1) umma_kernel(const __grid_constant__ CU
             const uint32_t tbase = tmem + (uint32_t)(ab * p.ncols) + ((uint32_t)(q * 32) << 16);
             for (int c0 = 0; c0 < ncol; c0 += 32) {
                 float v[32];
+                __syncwarp();                          // lanes past the last row skip the rest of the body
                 tmem_ld_32x32(tbase + (uint32_t)c0, v);
                 if (!rvalid) continue;
                 const int nbase = ti.n0 + c0;

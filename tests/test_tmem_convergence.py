@@ -58,7 +58,7 @@ def _loop_body(body, at):
             return i, j
 
 
-@pytest.mark.parametrize("name", ["conv_rows.cu", "conv_wgrad.cu"])
+@pytest.mark.parametrize("name", ["conv_rows.cu", "conv_wgrad.cu", "umma_gemm.cu"])
 def test_tmem_accesses_follow_a_meeting_of_the_warp(name):
     with open(os.path.join(CSRC, name)) as f:
         bodies = list(_kernels(f.read()))
