@@ -340,7 +340,9 @@ __global__ void __launch_bounds__(256) sirt_fp_slices_exact_kernel(SirtProblem q
 //     of the outer ones it has: a detector outside a pixel's window must not enter
 //     it, not even times zero (it may be infinite or NaN).
 // Both together took 16 slices x 10 iterations at N=512 / 360 angles from 10.4
-// to 9.2 ms against unshared windows gathered from global memory.
+// to 9.2 ms against unshared windows gathered from global memory (8.95 since the
+// third gather is chosen; two slices took 213 us per iteration with all three added
+// and take 217).
 // The update x + C*bp and both padded copies are the epilogue.  More than
 // kBpChunk angles keep their compensated totals in shared memory between
 // chunks.  `first`: block (0,0,0) applies the stopping rule of iteration it.
@@ -483,7 +485,12 @@ __global__ void __launch_bounds__(256, 4) sirt_bp_slices_kernel(SirtProblem q, i
                         f32x2 v0[V / 2], v1[V / 2], x[V / 2];
                         lds_pairs<V>(ad, v0);
                         lds_pairs<V>(ad + EB, v1);
-                        lds_pairs<V>(past ? ad + 2 * EB : ad, x);
+                        if constexpr (V == 4) {
+                            lds_pairs<V>(past ? ad + 2 * EB : ad, x);
+                        } else {                           // few blocks: the address is needed sooner than the value
+                            lds_pairs<V>(ad + 2 * EB, x);
+                            x[0] = past ? x[0] : v0[0];
+                        }
 #pragma unroll
                         for (int p = 0; p < V / 2; ++p) {
                             fa[p] = fma2(pk2(wF0, wF0), v0[p], fa[p]);
@@ -492,8 +499,8 @@ __global__ void __launch_bounds__(256, 4) sirt_bp_slices_kernel(SirtProblem q, i
                         const float wx = past ? wG2 : wG0;
 #pragma unroll
                         for (int p = 0; p < V / 2; ++p) {
-                            ga[p] = fma2(pk2(wx, wx), x[p], ga[p]);
                             ga[p] = fma2(pk2(wG1, wG1), v1[p], ga[p]);
+                            ga[p] = fma2(pk2(wx, wx), x[p], ga[p]);
                         }
                     }
                 };
