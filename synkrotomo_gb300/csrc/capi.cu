@@ -279,27 +279,47 @@ int valid_split(int s) { return s == 1 || s == 2 || s == 4 || s == 8; }
 // problem table is uploaded from it (a copy a CUDA graph can capture) instead
 // of from pageable memory.
 // Engine choice by the work per iteration (FP ray-row steps + BP pixel-angle
-// pairs), measured on GB300 on the same inputs.  One problem with deltarho 1:
+// pairs) and by the pixels of all slices, measured on GB300 on the same inputs.
+// One problem with deltarho 1:
 // - one slice up to kSmallSingle, and stacks up to kSmallStack: all iterations in
 //   one cooperative launch (sirt_small.cu, at most 360 angles).  us per
 //   iteration, there / two launches per iteration: N=64, 64 angles 8.9 / 12.7;
 //   N=128, 128 angles 12.9 / 17.8; N=256, 360 angles 62 / 76; N=512, 180 angles
 //   (1.1e8) 108 / 156; N=512, 360 angles (2.3e8) 189 / 273; N=768, 180 angles
 //   (2.6e8) 224 / 224; N=1024, 180 angles (4.6e8) 358 / 356.
-// - stacks above it: interleaved slices (sirt_slices.cu); there / one launch:
-//   N=96, 90 angles, 16 slices (3.2e7) 66 / 50; N=256, 180 angles, 2 slices
-//   (5.7e7) 81 / 61; N=256, 60 angles, 8 slices (7.6e7) 76 / 91; N=64, 64 angles,
-//   128 slices (8.1e7) 77 / 111.
-// Otherwise (other spacings, more angles, engine forced, several problems):
+// - stacks above it with 1280 pixels for each SM (1.25 tiles of 32 x 32; 1024 for
+//   slices of up to 64 pixels a side): interleaved slices (sirt_slices.cu), whose
+//   backward phase walks all angles of a tile in one block, about 0.25 us each
+//   however few the tiles are.  There / one launch: N=256, 180 angles, 2
+//   slices (5.7e7) 81 / 61; N=256, 60 angles, 8 slices (7.6e7) 76 / 91; N=64, 64
+//   angles, 128 slices (8.1e7) 77 / 111.  There / angles split over warps (the
+//   projector's forward grid and the generic backward phase): N=96, 600 angles, 8
+//   slices (485 pixels an SM) 198 / 102; N=96, 600 angles, 16 slices (970) 214 /
+//   177; N=192, 361 angles, 4 slices (970) 139 / 118; N=128, 360 angles, 10 slices
+//   (1078) 150 / 130; N=160, 361 angles, 8 slices (1347) 146 / 160; N=256, 360
+//   angles, 4 slices (1725) 155 / 179; N=64, 360 angles, 32 / 40 / 52 slices (862 /
+//   1078 / 1401) 141 / 123, 149 / 145, 150 / 172; N=32, 360 angles, 100 / 160
+//   slices (674 / 1078) 144 / 124, 158 / 182.  Slices of up to 64 pixels a side
+//   leave many lanes of the one launch's units idle, so they go over from
+//   kSmallNarrow on: N=32, 30 angles, 500 slices (3.7e7) 64 / 135; N=64, 45 angles,
+//   100 slices (4.5e7) 56 / 69; N=64, 60 angles, 52 slices (3.1e7) 53 / 51; but
+//   N=128, 60 angles, 16 slices (3.8e7) 58 / 50, N=256, 60 angles, 4 slices (3.8e7)
+//   59 / 45.
+// Otherwise (other spacings, more angles, few pixels, engine forced, several problems):
 // - up to kSmallWork the phase-split engine with the generic forward phase
 //   (two launches per iteration, no grid barrier) beats the persistent kernel
 //   1.08-1.32x (N=64-256, 1-64 slices);
 // - above it, for one problem, the split engine whose forward phase runs on
 //   the projector's own grid beats it 1.04-1.16x (N=256-1024, 1-256 slices;
 //   N=2048 / 1 slice even); batches of several problems keep the persistent
-//   kernel there.
+//   kernel there.  Its backward phase runs on the backprojector's tiles (32 x 64
+//   pixels) where they give the SMs 7/4 blocks each, else in the generic phase,
+//   which splits the angles: one slice of 1000 angles, tiles / generic, N=576 667 /
+//   483, N=704 (242 blocks) 758 / 699, N=768 (288) 816 / 851, N=1024 1271 / 1412;
+//   N=128, 600 angles, 4 slices 308 / 96.
 constexpr double kSmallWork = 6.0e7;
 constexpr double kSmallStack = 6.5e7;
+constexpr double kSmallNarrow = 3.0e7;
 constexpr double kSmallSingle = 2.5e8;
 
 int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double tol, int grid_blocks,
@@ -346,7 +366,11 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
     if (split && !sirt_phase_grids(&fpg, &bpg)) return fail(ctx, SYNK_ECUDA, "SIRT phase kernels cannot be resident");
     // a stack of slices: both phases on interleaved slices, the geometry evaluated once per group of them
     const bool fits = split && nprob == 1 && in[0].nslices <= 65535 && (in[0].a + 31) / 32 + 2 <= 65535;
-    const bool slices = fits && in[0].nslices >= 2 && work > kSmallStack && in[0].deltarho == 1.0f &&
+    const long long sms = device_sms(), side = (in[0].size + 31) / 32;
+    const bool narrow = in[0].size <= 64;
+    const bool slices = fits && in[0].nslices >= 2 && work > (narrow ? kSmallNarrow : kSmallStack) &&
+                        (long long)in[0].nslices * in[0].size * in[0].size >= (narrow ? 1024 : 1280) * sms &&
+                        in[0].deltarho == 1.0f &&
                         slices_fit(make_geom(in[0].a, in[0].rhozero, in[0].deltarho, in[0].numrhos, in[0].size,
                                              nullptr));
     // one small problem (or stack): every iteration in one cooperative launch
@@ -403,8 +427,8 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         SYNK_CUDA(sc.get(&R, pr), "cudaMallocAsync(R)");
         SYNK_CUDA(sc.get(&C, n), "cudaMallocAsync(C)");
         // slices: xpad, xTpad and rr hold interleaved slice groups
-        const size_t npx = slices ? slices_floats(np, q.nslices) : np * q.nslices + (small ? 8 : 0);
-        const size_t nrr = slices ? slices_floats(pr, q.nslices) : pr * q.nslices;
+        const size_t npx = slices ? slices_floats(np, q.nslices, q.size) : np * q.nslices + (small ? 8 : 0);
+        const size_t nrr = slices ? slices_floats(pr, q.nslices, q.size) : pr * q.nslices;
         SYNK_CUDA(sc.get(&xpad, npx), "cudaMallocAsync(padded image)");
         SYNK_CUDA(sc.get(&xTpad, npx), "cudaMallocAsync(padded transposed image)");
         SYNK_CUDA(sc.get(&rr, nrr), "cudaMallocAsync(residual)");
@@ -419,7 +443,7 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         // the backprojection-grid backward phase (one large problem, every
         // window of its 64-row tiles in range) reads rr as detector pairs
         float *rrp = nullptr;
-        if (stack && !slices && bp_windows_in_range(h.P, 64)) {
+        if (stack && !slices && 4 * q.nslices * side * ((q.size + 63) / 64) >= 7 * sms && bp_windows_in_range(h.P, 64)) {
             SYNK_CUDA(sc.get(&rrp, 2 * pr * q.nslices), "cudaMallocAsync(residual pairs)");
             SYNK_CUDA(cudaMemsetAsync(rrp, 0, sizeof(float) * 2 * pr * q.nslices, st), "memset");
         }

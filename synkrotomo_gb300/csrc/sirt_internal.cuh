@@ -87,7 +87,7 @@ cudaError_t launch_sirt_fp_stack(const SirtProblem &q, int it, double tol2, int 
 cudaError_t launch_sirt_bp_stack(const SirtProblem &q, int it, double tol2, int *active, cudaStream_t stream);
 // slice groups (sirt_slices.cu): both phases of a stack of at least two slices with deltarho 1 on interleaved
 // slices (xpad, xTpad and rr of the problem hold the groups); want_e2: the residual sums are read (tol or history)
-size_t slices_floats(size_t per_slice, int nslices);   // floats of a group buffer with per_slice entries a slice
+size_t slices_floats(size_t per_slice, int nslices, int N);   // floats of a group buffer with per_slice entries a slice of side N
 bool slices_fit(const ProbGeom &P);                     // 32-bit offsets suffice
 cudaError_t launch_slices_load(const float *x, float *xs, float *xTs, int N, int nslices, cudaStream_t stream);
 cudaError_t launch_slices_store(float *xs, float *x, int N, int nslices, cudaStream_t stream);
