@@ -295,8 +295,8 @@ int valid_split(int s) { return s == 1 || s == 2 || s == 4 || s == 8; }
 //   angles, 128 slices (8.1e7) 77 / 111.  There / angles split over warps (the
 //   projector's forward grid and the generic backward phase): N=96, 600 angles, 8
 //   slices (485 pixels an SM) 198 / 102; N=96, 600 angles, 16 slices (970) 214 /
-//   177; N=192, 361 angles, 4 slices (970) 139 / 118; N=128, 360 angles, 10 slices
-//   (1078) 150 / 130; N=160, 361 angles, 8 slices (1347) 146 / 160; N=256, 360
+//   177; N=192, 361 angles, 4 slices (970) 139 / 118; N=128, 361 angles, 8 slices
+//   (862) 136 / 112; N=160, 361 angles, 8 slices (1347) 146 / 160; N=256, 360
 //   angles, 4 slices (1725) 155 / 179; N=64, 360 angles, 32 / 40 / 52 slices (862 /
 //   1078 / 1401) 141 / 123, 149 / 145, 150 / 172; N=32, 360 angles, 100 / 160
 //   slices (674 / 1078) 144 / 124, 158 / 182.  Slices of up to 64 pixels a side

@@ -468,18 +468,27 @@ static int fp_row_split(long long warps) {
 
 // Angle count from which fp_lane_kernel runs.  Below it neighbouring angles lie so
 // far apart that a warp of 4 angles walks rows and reads lines its lanes share
-// little of.  Lane / detector kernel, us per call: N=2048, 64 angles 566 / 215;
-// N=1024, 95 angles 177 / 97; N=512, 95 angles 55 / 48; N=512, 180 angles 68 / 71;
-// N=2048, 256 angles 578 / 646.
+// little of.  Lane / detector kernel, us per call: N=2048, 96 angles 348 / 260, 159
+// angles 423 / 365; N=1024, 96 angles 100 / 77, 159 angles 126 / 106; N=512, 96
+// angles 49 / 32, 159 angles 57 / 41; N=256, 159 angles 25 / 22; N=128, 140 angles
+// 15.6 / 14.5, 159 angles 15.6 / 15.4, 170 angles 16.1 / 16.1, 256 angles 17.5 /
+// 19.0.  From 256 pixels a side on the two meet later (N=512, 200 angles 65 / 50, 256
+// angles 66 / 59; N=1024 and N=2048, 256 angles 159 / 159 and 565 / 550).
 constexpr int kFpDetAngles = 160;
 
 static void launch_fp_rays(const ProbGeom &P, const AngleLists &L, const PairImages &X, float *sino,
                            cudaStream_t stream) {
     if (P.a < kFpDetAngles) {
-        // angle slots: the padded groups of 32 of both classes; rows split to >= 16 a part
+        // angle slots: the padded groups of 32 of both classes; rows split to >= 16 a
+        // part, beyond 8 parts only while a part's chain of gathers and not the warps'
+        // start-up bounds the call (about 116 warps for each SM): N=512, 4 angles 20
+        // us with 8 parts, 15 with 32; 30 angles 22 / 23, 21 with 16; 96 angles 32 / 41;
+        // 96 angles at a quarter of the pitch 76 / 118; N=2048, 159 angles 365 / 419
+        const int dgroups = (P.D + 31) / 32;
+        const long long warps = (long long)P.a * dgroups;
         int S = 1;
         while (S < 32 && P.N / (2 * S) >= 16) S *= 2;
-        const int dgroups = (P.D + 31) / 32;
+        while (S > 8 && warps * S > 116LL * device_sms()) S /= 2;
         const dim3 grid((dgroups + 32 / S - 1) / (32 / S), ((P.a + 31) / 32 + 1) * 32);
         switch (S) {
             case 1: fp_det_kernel<1><<<grid, 1024, 0, stream>>>(P, L, X.base, X.plane, X.cls, sino); break;
