@@ -385,7 +385,12 @@ __global__ void __launch_bounds__(256, 5) fp_lane_kernel(ProbGeom P, AngleLists 
     }
     const int rr = r < P.D ? r : P.D - 1;          // keep every warp for the block reduction
     const int jb = part * P.N / S, je = (part + 1) * P.N / S;
-    float v = fp_lane_ray_pair(P, r < P.D ? k : -1, rr, base, flat ? plane : 0u, jb, je);
+    float v = 0.0f;
+    // a warp whose detectors all lie past the image sets up no line (N=16, 2000 angles,
+    // 3000 detectors 46 -> 33 us; N=2048, 2048 angles 3.10 -> 3.02 ms)
+    const float rho = __fadd_rn(P.rhozero, __fmul_rn((float)rr, P.deltarho));
+    if (S > 1 || __any_sync(0xffffffffu, !(fabsf(rho) > 0.75f * (float)P.N + 2.0f)))
+        v = fp_lane_ray_pair(P, r < P.D ? k : -1, rr, base, flat ? plane : 0u, jb, je);
     if (S > 1) {
         red[warp][lane] = v;
         __syncthreads();

@@ -1,6 +1,7 @@
 """Row parts of the forward projector's detector kernel (csrc/project.cu,
 launch_fp_rays), by the kernel names that the profiler records, and its values
 against the FP32 restatement: the parts shrink from 32 to 8 as the rays grow.
+And the lane kernel's warps whose detectors lie past the image.
 
 Tolerances: the projector's parity bar, 1e-5 relative L2, and 1e-4 of the largest
 value per ray."""
@@ -35,3 +36,18 @@ def test_row_parts(gpu, size, angles, deltarho, kernel):
     assert rel_l2(out, ref) < 1e-5
     assert np.max(np.abs(out - ref)) <= 1e-4 * max(1.0, float(np.max(np.abs(ref))))
     assert any(kernel in n for n in _kernels(lambda: rt.forwardprojection(*args)))
+
+
+@pytest.mark.parametrize("size,angles,det,first", [(16, 200, 300, -150.0), (34, 161, 90, 20.0), (66, 170, 47, -800.0)])
+def test_detectors_past_the_image(gpu, size, angles, det, first):
+    """Rows that reach far past the image on both sides, on one, and not to it at all
+    (those rays must be zero)."""
+    ang = phantom.geometry(size, angles).angles
+    img = np.random.default_rng(size).random(size * size).astype(np.float32)
+    out = rt.forwardprojection(torch.from_numpy(ang).cuda(), first, 1.0, det, torch.from_numpy(img).cuda()).cpu().numpy()
+    ref = cpu_ref.forwardprojection(ang, first, 1.0, det, img)
+    if first == -800.0:
+        assert not ref.any() and not out.any()
+    else:
+        assert rel_l2(out, ref) < 1e-5
+        assert np.max(np.abs(out - ref)) <= 1e-4 * max(1.0, float(np.max(np.abs(ref))))
