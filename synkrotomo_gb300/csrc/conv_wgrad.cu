@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(192, 1) conv_wgrad_kernel(const __grid_constan
     constexpr uint32_t kM = CI == 64 ? 2 : 1;            // MMAs of M = 128 that hold the three taps kx
     constexpr int kLate = (2 + R - 1) / R;               // steps for which a gradient row is used again
     extern __shared__ uint8_t smem_raw[];
+    __shared__ float sdb[4][CO];                         // the warps' bias sums
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *zs = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     const int S = p.stages;
@@ -332,18 +333,23 @@ __global__ void __launch_bounds__(192, 1) conv_wgrad_kernel(const __grid_constan
                 if (lane == 0) mbar_arrive(tempty);
             }
         }
-        if (bias && ok) {
+        if (bias) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                float a = acc[e];
+                float a = ok ? acc[e] : 0.0f;
 #pragma unroll
                 for (uint32_t o = kG; o < 32u; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-                if (r0 == 0u) atomicAdd(p.db + co0 + 8u * c + e, a);
+                if (r0 == 0u) sdb[q4][8u * c + e] = a;
             }
         }
     }
     tc_fence_before();
     __syncthreads();
+    // one atomic per CTA and channel: their rounding is most of the sum's (32 images,
+    // positive terms: 6.4e-8 of the sum from 64 bits, 4.8e-7 with one per warp)
+    if (bias && threadIdx.x < CO)
+        atomicAdd(p.db + co0 + threadIdx.x,
+                  (sdb[0][threadIdx.x] + sdb[1][threadIdx.x]) + (sdb[2][threadIdx.x] + sdb[3][threadIdx.x]));
     if (warp == 0) {
         tc_fence_after();
         tmem_dealloc(tmem, 512u);
@@ -358,14 +364,16 @@ static cudaError_t dw_launch(const DwArgs &a, DwParams &p, cudaStream_t st) {
     p.rows = (long long)a.B * p.tiles_w * a.H;
     if (p.rows == 0) return cudaSuccess;
     const int chunks = a.Cin / CI, cols = (CI == 64 ? 2 : 1) * 3 * CO;
-    // While the rows are few a CTA takes as many input blocks as the 512 TMEM columns
-    // hold, so that a gradient strip is read for all of them, and all SMs work.  The
-    // tensor cores' FP32 sums cut off below their last bit at every step, 2^-25 of
-    // the sum on average.  Where the rows are many (full-resolution layers of 12 and
-    // more images) the cut-off bits that shorter sums do not lose would move the
-    // gradient by up to 2.1e-5 of its norm from what it was with one tap per CTA and
-    // 33 parts (3970 steps a sum at 32 images): there 40 parts of one block each, 3277
-    // steps.
+    // All SMs work, and while the rows are few a CTA takes as many input blocks as the
+    // 512 TMEM columns hold, so that a gradient strip is read for all of them.  The
+    // tensor cores' FP32 sums cut off below their last bit at every step, so a sum is
+    // the more exact the shorter it is.  Full-resolution layers of 12 and more images:
+    // at most 40 parts of one block each took the training step of 32 images 3.59 ms,
+    // and the last layer's weight gradient was 6.3e-5 of its absolute sum from 64
+    // bits; as many parts as SMs take 3.26 ms and are 9.7e-6 from it.  (All blocks in
+    // one CTA there too: another 25 us less, but the 96 -> 32 layer's shorter sums would
+    // move the whole gradient by more than the 2e-5 of its norm that one version may
+    // differ from the next.)
     const bool many = CI == 32 && CO == 32 && p.rows > 6144;
     p.nc = 1;
     if (!many)
@@ -373,10 +381,9 @@ static cudaError_t dw_launch(const DwArgs &a, DwParams &p, cudaStream_t st) {
     p.nci = chunks / p.nc;
     p.nco = a.Cout / CO;
     const int nblk = p.nci * p.nco, sms = device_sms();
-    long long want = nblk < sms ? sms / nblk : 1;
-    if (many && want > 40) want = 40;
+    const long long want = nblk < sms ? sms / nblk : 1;
     p.splits = (int)(want < p.rows ? want : p.rows);
-    // nor does any sum cover more than a sixteenth of the pixels
+    // no sum covers more than a sixteenth of the pixels
     p.turns = (16 + p.splits - 1) / p.splits;
     p.x_tx = (uint32_t)(R * (PX + 2) * 2 * CI);
     p.z_tx = (uint32_t)(R * PX * 2 * CO);
