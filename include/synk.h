@@ -18,8 +18,10 @@
  *    reference's f32 / i32 types.
  *  - Entry points are stream-ordered: they enqueue work on the context's
  *    stream and return launch/validation errors.  Errors that happen while
- *    the GPU runs (a persistent kernel's grid barrier that timed out) are
- *    reported by the next synk_context_sync().
+ *    the GPU runs (a wait inside a kernel that ran out: see
+ *    synk_context_set_barrier_limit) leave an invalid result and are reported
+ *    by the next synk_context_sync() only: a caller that never calls it does
+ *    not learn of them.
  *  - Inputs are never modified.  Scratch memory is taken from CUDA's
  *    stream-ordered allocator (cudaMallocAsync) on the context's stream.
  *  - A context is used by one host thread at a time.
@@ -41,7 +43,7 @@ extern "C" {
 #define SYNK_OK 0
 #define SYNK_EINVAL 1    /* bad argument (shape, size, null pointer)       */
 #define SYNK_ECUDA 2     /* a CUDA runtime call failed                     */
-#define SYNK_ETIMEOUT 3  /* a persistent kernel's grid barrier timed out   */
+#define SYNK_ETIMEOUT 3  /* a wait inside a kernel ran out of time         */
 #define SYNK_ENOMEM 4    /* device allocation failed                       */
 
 typedef struct synk_context synk_context;
@@ -54,15 +56,19 @@ int synk_context_new(synk_context **out, int device, void *stream);
 void synk_context_free(synk_context *ctx);
 /* Redirects subsequent work to another stream of the same device. */
 int synk_context_set_stream(synk_context *ctx, void *stream);
-/* Waits for the context's stream; returns SYNK_ETIMEOUT if a persistent
- * kernel gave up at a grid barrier, SYNK_ECUDA on an asynchronous CUDA error. */
+/* Waits for the context's stream; returns SYNK_ETIMEOUT if a kernel gave up at
+ * a wait (its result is invalid), SYNK_ECUDA on an asynchronous CUDA error. */
 int synk_context_sync(synk_context *ctx);
-/* Time limit of every wait inside the library's persistent kernels (the SIRT
- * grid barrier, the tensor-core engine's mbarrier waits): default 2 s, range
- * [1 us, 60 s].  A wait that runs out records SYNK_ETIMEOUT, its kernel
- * returns, and the next synk_context_sync() reports it and clears it.
+/* Time limit of every wait inside the library's kernels: the grid barriers of
+ * the two SIRT engines that run all iterations in one cooperative launch (the
+ * persistent kernel of batches, and one small problem, which is what a plain
+ * synk_SIRT of up to 360 angles runs: see grid_blocks) and the tensor-core
+ * engine's mbarrier waits.  Default 2 s, range [1 us, 60 s].  A wait that runs
+ * out records SYNK_ETIMEOUT, its kernel returns with an invalid result, and the
+ * next synk_context_sync() reports it and clears it.  Time in which the GPU ran
+ * another process does not count in the small problem's barrier.
  * missing_blocks > 0 is fault injection for testing that path: the grid
- * barrier of the next persistent SIRT launches waits for that many blocks
+ * barrier of the next such SIRT launches waits for that many blocks
  * more than were launched, so every barrier runs out after timeout_ns.  Pass
  * 0 in production.  No reference counterpart: the reference surfaces failures
  * only as the runtime's error codes (futhark's context error string). */
@@ -127,25 +133,26 @@ typedef struct synk_sirt_options {
     int32_t fp_split;
     int32_t bp_split;
     /* Engine and grid: > 0 = the persistent kernel with that many blocks;
-     * 0 = automatic (one launch per phase and iteration for a single problem,
-     * and for batches whose iteration is small: at most 6e7 ray-row steps plus
-     * pixel-angle pairs; otherwise the persistent kernel with every block that
-     * fits); -1 = one launch per phase and iteration.  With tol > 0 the
-     * launch loop ends early: every 16 iterations the call reads the number of
+     * 0 = automatic (a single problem with deltarho 1 and at most 360 angles runs
+     * in one cooperative launch up to 2.5e8 ray-row steps plus pixel-angle pairs
+     * per iteration, 6.5e7 for a stack; other single problems, and batches of at
+     * most 6e7, one launch per phase and iteration; larger batches the persistent
+     * kernel with every block that fits); -1 = one launch per phase and
+     * iteration.  With tol > 0 the launch loop ends early: every 16 iterations the call reads the number of
      * slices still updating, which waits for the stream (not while the stream
      * is being captured into a graph; the loop then runs to the end, each
      * launch doing nothing once every slice has stopped). */
     int32_t grid_blocks;
 } synk_sirt_options;
 
-/* SIRT of `nslices` independent slices sharing one geometry in ONE persistent
- * launch: image/out/projections hold nslices consecutive slices ([nslices*n]
+/* SIRT of `nslices` independent slices sharing one geometry in one call:
+ * image/out/projections hold nslices consecutive slices ([nslices*n]
  * and [nslices*p]); image may be NULL for a zero start. */
 int synk_sirt_slices(synk_context *ctx, float *out, const float *angles, int64_t a, float rhozero,
                      float deltarho, int32_t numrhos, int32_t size, int32_t nslices, const float *image,
                      const float *projections, int32_t iterations, const synk_sirt_options *opts);
 
-/* Independent SIRT problems of any sizes in ONE persistent launch (no
+/* Independent SIRT problems of any sizes in one call (no
  * reference counterpart; SIRT3D is the special case of one problem with many
  * slices).  Each problem is a stack of `nslices` slices sharing one geometry.
  * All arrays are device pointers: image [nslices*size*size] (NULL = zero

@@ -33,7 +33,7 @@ struct synk_context {
     int device = 0;
     cudaStream_t stream = nullptr;
     std::string err;
-    int *d_status = nullptr;   // written by persistent kernels (SYNK_ETIMEOUT)
+    int *d_status = nullptr;   // written by kernels whose waits ran out (SYNK_ETIMEOUT)
     int *h_poll = nullptr;     // pinned: active-slice counts read back by the SIRT loop's stopping rule
     cudaEvent_t poll_ev[2] = {nullptr, nullptr};
     unsigned long long barrier_timeout_ns = 2000000000ull;
@@ -709,7 +709,7 @@ int synk_context_sync(synk_context *ctx) {
     if (status != SYNK_OK) {
         cudaMemset(ctx->d_status, 0, sizeof(int));
         if (status == SYNK_ETIMEOUT)
-            return fail(ctx, SYNK_ETIMEOUT, "a grid barrier of the persistent SIRT kernel timed out; the result is invalid");
+            return fail(ctx, SYNK_ETIMEOUT, "a wait inside a kernel (a SIRT grid barrier, a tensor-core mbarrier) timed out; the result is invalid");
         return fail(ctx, status, "device status %d", status);
     }
     return SYNK_OK;

@@ -2,10 +2,12 @@
 // in plain integers so that a host test can evaluate them.
 #pragma once
 
+#ifndef SYNK_HD
 #ifdef __CUDACC__
 #define SYNK_HD __host__ __device__ __forceinline__
 #else
 #define SYNK_HD inline
+#endif
 #endif
 
 namespace synk {

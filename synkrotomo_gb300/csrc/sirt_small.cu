@@ -31,6 +31,7 @@
 #include "sirt_internal.cuh"
 #include "sirt_device.cuh"
 #include "sirt_offset.cuh"
+#include "poll_limit.cuh"
 #include "fp_tile.cuh"
 #include "bp_tile.cuh"
 
@@ -76,7 +77,7 @@ __device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned *p) {
 }
 
 // Grid barrier number `epoch` (1, 2, ...): the counter only grows.  False in
-// every thread once the wait ran out of time (the status word is then set).
+// every thread once the wait ran out of time (PollLimit; the status word is then set).
 __device__ __forceinline__ bool small_barrier(unsigned *count, unsigned target, int *status,
                                               unsigned long long timeout_ns, int *s_flag) {
     __syncthreads();
@@ -84,9 +85,10 @@ __device__ __forceinline__ bool small_barrier(unsigned *count, unsigned target, 
         int ok = 1;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
         if ((int)(ld_relaxed_u32(count) - target) < 0) {
-            const unsigned long long t0 = global_ns();
+            PollLimit limit;
+            limit.start(global_ns());
             for (unsigned spin = 1; (int)(ld_relaxed_u32(count) - target) < 0; ++spin)
-                if ((spin & 63u) == 0u && (global_ns() - t0 > timeout_ns || spin > (1u << 30))) {
+                if ((spin & 63u) == 0u && (limit.over(global_ns(), timeout_ns) || spin > (1u << 30))) {
                     atomicExch(status, SYNK_ETIMEOUT);
                     ok = 0;
                     break;

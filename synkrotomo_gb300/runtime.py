@@ -59,7 +59,8 @@ class _Context:
         self.check(rc, "synk_context_sync")
 
     def set_barrier_limit(self, timeout_ns: int = 2_000_000_000, missing_blocks: int = 0):
-        """Time limit of the persistent kernels' waits; ``missing_blocks`` > 0
+        """Time limit of the waits inside kernels (the grid barriers of the SIRT
+        engines that run in one launch, the tensor cores' mbarriers); ``missing_blocks`` > 0
         injects a barrier that waits for blocks that never arrive (testing
         the SYNK_ETIMEOUT path; 0 in production)."""
         self.check(self.lib.synk_context_set_barrier_limit(self.handle, int(timeout_ns), int(missing_blocks)),
@@ -165,6 +166,7 @@ class DeviceArray:
         self._ctx = ctx
 
     def torch(self) -> torch.Tensor:
+        """The device tensor, without waiting (and so without ``get()``'s check)."""
         return self._t
 
     def get(self) -> np.ndarray:
@@ -226,7 +228,8 @@ def sirt_slices(angles: torch.Tensor, rhozero: float, deltarho: float, numrhos: 
                 image: torch.Tensor | None, projections: torch.Tensor, iterations: int, tol: float = 0.0,
                 residuals: bool = False, fp_split: int = 0, bp_split: int = 0, grid_blocks: int = 0,
                 out: torch.Tensor | None = None):
-    """SIRT of ``nslices`` independent slices in one persistent launch.
+    """SIRT of ``nslices`` independent slices.  Returns without waiting: a
+    kernel's wait that ran out of time is reported by ``context().sync()``.
 
     Returns ``(x, res, done)``: x [nslices*size*size]; res [nslices,
     iterations+1] relative residuals ||FP(x_k)-b||/||b|| (float64, None unless
@@ -284,7 +287,7 @@ def resident_blocks() -> int:
 
 
 def sirt_batch(problems: list, tol: float = 0.0, grid_blocks: int = 0) -> list:
-    """Every problem's SIRT in one persistent launch (``synk_sirt_batch``);
+    """Every problem's SIRT in one call (``synk_sirt_batch``);
     results land in each problem's ``out`` / ``residuals`` / ``done``."""
     if not problems:
         return problems
@@ -327,7 +330,9 @@ class SirtPlan:
 
 def sirt(angles: torch.Tensor, rhozero: float, deltarho: float, image: torch.Tensor, projections: torch.Tensor,
          iterations: int, out: torch.Tensor | None = None) -> torch.Tensor:
-    """``iterations`` SIRT updates from ``image`` (futhark/SIRT.fut:43-49)."""
+    """``iterations`` SIRT updates from ``image`` (futhark/SIRT.fut:43-49).
+    Returns without waiting: a kernel's wait that ran out of time is reported by
+    ``context().sync()``."""
     ctx = context(projections.device.index)
     if out is None:
         out = torch.empty(image.numel(), dtype=torch.float32, device=projections.device)
