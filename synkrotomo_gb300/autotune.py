@@ -1,4 +1,4 @@
-"""Autotuner of the persistent SIRT kernel's launch shape.
+"""Autotuner of the launched SIRT engines' shapes.
 
 Tunables per problem:
   fp_split     1/2/4/8 warps share one ray of the forward phase (rows split);
@@ -10,7 +10,9 @@ Tunables per problem:
 Each candidate is timed on the problem itself (a few iterations, CUDA events);
 the winner is cached in a JSON file keyed by the size bucket
 (image side, angle count, detector count, slices rounded to powers of two), so
-a bucket is measured once per machine.  Cache file: $SYNK_TUNE_CACHE, else
+a bucket is measured once per machine.  The library's own choice (no shape given:
+grid_blocks 0, which alone reaches the engine that runs a small problem in one
+launch) is timed beside it; ``launch_kwargs`` gives whichever was faster.  Cache file: $SYNK_TUNE_CACHE, else
 ~/.cache/synkrotomo_gb300/autotune.json.
 """
 from __future__ import annotations
@@ -86,9 +88,37 @@ def choose(key: str, cands: list, measure, cache: dict | None = None, path: str 
         return best
 
 
+DEFAULT = dict(fp_split=0, bp_split=0, grid_blocks=0)     # the library's own choice
+
+
+def with_default(key: str, choice: dict, measure, path: str | None = None) -> dict:
+    """``choice`` with the time of the library's own choice, ``default_ms``,
+    measured and stored where the cached entry has none (entries of versions that
+    did not time it)."""
+    if "default_ms" in choice:
+        return choice
+    choice = dict(choice, default_ms=measure(dict(DEFAULT)) * 1e3)
+    with _lock:
+        cache = load_cache(path)
+        cache[key] = choice
+        save_cache(cache, path)
+    return choice
+
+
+def launch_kwargs(choice: dict) -> dict:
+    """Arguments of ``sirt_slices`` / the problem options for a tuned choice: its
+    shape, or the library's own choice where that was at least as fast."""
+    if choice.get("default_ms", float("inf")) <= choice.get("ms", 0.0):
+        return dict(DEFAULT)
+    return {k: int(choice[k]) for k in DEFAULT}
+
+
 def tune_sirt(angles, rhozero: float, deltarho: float, numrhos: int, size: int, projections, nslices: int = 1,
               iterations: int = 6, path: str | None = None) -> dict:
-    """Tuned launch shape for SIRT of this geometry (measured on the GPU)."""
+    """Tuned launch shape for SIRT of this geometry (measured on the GPU), with the
+    times of it (``ms``) and of the library's own choice (``default_ms``).  Solve with
+    ``**launch_kwargs(choice)``: the shape alone can be slower than no shape (N=128,
+    128 angles: 17.8 us per iteration against 12.9)."""
     import torch
 
     from . import _lib
@@ -113,4 +143,4 @@ def tune_sirt(angles, rhozero: float, deltarho: float, numrhos: int, size: int, 
         torch.cuda.synchronize()
         return e0.elapsed_time(e1) * 1e-3
 
-    return choose(key, candidates(size, angles.numel(), resident), measure, path=path)
+    return with_default(key, choose(key, candidates(size, angles.numel(), resident), measure, path=path), measure, path)
