@@ -1,11 +1,12 @@
-// Pixel-driven backprojection of a tile, shared by the standalone
-// backprojector and the persistent SIRT kernel.
+// Pixel-driven backprojection of a tile: bp_chunk_pair on rows of detector pairs
+// (the standalone backprojector, SIRT of one large slice), bp_chunk on plain rows
+// (the persistent and phase SIRT kernels, the backprojector without scratch).
 //
-// A block of 256 threads owns a tile of 32 columns; thread (lane, warp) owns
-// column lane and PIX rows spaced RSTEP apart.  The per-angle constants of
-// the chord-length trapezoid are staged in shared memory kBpChunk angles at a time
-// and read as one broadcast float4 + one float2 per angle; each (pixel, angle)
-// then costs ~14 FP32/INT instructions and two sinogram gathers:
+// A block of 256 threads owns a tile of 32 columns; a thread owns one column and
+// PIX rows spaced apart.  The per-angle constants of the chord-length trapezoid are
+// staged in shared memory kBpChunk angles at a time and read as one broadcast
+// float4 + one float2 per angle; each (pixel, angle) then costs 9-10 warp
+// instructions with one 8-byte gather, or ~14 with two 4-byte ones:
 //   q    = x_c*cos - y_c*sin - rz_c               (rho of the centre from the middle
 //                                                  detector position rz_c, ProbGeom)
 //   s0   = ceil((q - sqrt(2)/2) / deltarho) + zi  (first candidate detector)
@@ -333,7 +334,5 @@ __device__ __forceinline__ void bp_exact_angles(const ProbGeom &P, const int *__
         }
     }
 }
-
-cudaError_t launch_exact_list(const ProbGeom &P, int *list, int *count, cudaStream_t stream);
 
 }  // namespace synk

@@ -413,7 +413,7 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         int2 *graze, *graze_tmp;
         float *glen_tmp;
         // rays that only clip a corner pixel: per corner and angle at most
-        // ceil(1/deltarho) + 1 (graze_list_kernel)
+        // ceil(1/deltarho) + 1 (rownorm_kernel)
         const double gcapc = (double)q.a * (ceil(1.0 / (double)q.deltarho) + 1.0);
         const int graze_capc = (int)std::max(1.0, std::min({gcapc, (double)pr, (double)(1 << 26)}));
         SYNK_CUDA(sc.get(&geom, (size_t)q.a), "cudaMallocAsync");

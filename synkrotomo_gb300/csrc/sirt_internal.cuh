@@ -56,7 +56,9 @@ struct SirtParams {
     int dynamic;          // hand out items with an atomic counter (uneven batches)
 };
 
-// One small problem in one cooperative launch (sirt_small.cu): deltarho 1, at most kSirtSmallAngles angles.
+// One small problem in one cooperative launch (sirt_small.cu): deltarho 1, at most
+// kSirtSmallAngles angles, whose constants fit beside the warps' ray tables in the 48
+// KB of static shared memory.
 constexpr int kSirtSmallAngles = 360;
 struct SirtSmall {
     SirtProblem q;

@@ -66,7 +66,6 @@ struct SmallShared {
     int4 unit[kWarpsSmall];
     float4 line[kWarpsSmall][32], meas[kWarpsSmall][32];
     float red[kWarpsSmall][33];
-    double e2[kWarpsSmall];
     int flag, any;
 };
 

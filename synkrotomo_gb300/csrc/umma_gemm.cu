@@ -39,7 +39,6 @@ using namespace umma;
 __device__ __forceinline__ uint16_t f2bf(float x) {
     return __bfloat16_as_ushort(__float2bfloat16_rn(x));
 }
-__device__ __forceinline__ float bf2f(uint16_t x) { return __bfloat162float(__ushort_as_bfloat16(x)); }
 
 // The coordinates of one output tile (linear index t over gx x gy x gz).
 struct TileInfo {
