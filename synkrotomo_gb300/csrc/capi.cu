@@ -264,6 +264,8 @@ __global__ void fill_i32_kernel(int *p, int n, int v) {
     if (i < n) p[i] = v;
 }
 
+__global__ void store_problem_kernel(SirtProblem q, SirtProblem *dst) { *dst = q; }
+
 int pick_fp_split(long long tasks, long long resident_warps, int size) {
     const int maxs = size / 16 > 8 ? 8 : (size / 16 < 1 ? 1 : size / 16);
     return pick_split(tasks, resident_warps, maxs);
@@ -533,11 +535,18 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
     SYNK_CUDA(sc.get(&dprobs, (size_t)nprob), "cudaMallocAsync(problem table)");
     SYNK_CUDA(sc.get(&totals, 2), "cudaMallocAsync");
     SYNK_CUDA(sc.get(&words, 8), "cudaMallocAsync");
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cap = cudaStreamCaptureStatusNone;
     if (staging) {
         // pinned copy: stays valid for every replay of a captured graph
         memcpy(staging, sorted.data(), sizeof(SirtProblem) * nprob);
         SYNK_CUDA(cudaMemcpyAsync(dprobs, staging, sizeof(SirtProblem) * nprob, cudaMemcpyHostToDevice, st),
                   "upload problem table");
+    } else if (cap != cudaStreamCaptureStatusNone) {
+        // the caller captures this stream: a copy node would read the host vector at
+        // every replay, when it is gone; a kernel's arguments are kept in the graph
+        for (int i = 0; i < nprob; ++i) store_problem_kernel<<<1, 1, 0, st>>>(sorted[i], dprobs + i);
+        SYNK_CUDA(cudaGetLastError(), "upload problem table");
     } else {
         // from pageable memory: the copy is staged before the call returns, so
         // the host vector may go out of scope afterwards
@@ -578,8 +587,6 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         int *active = reinterpret_cast<int *>(words + 7);
         // the early exit reads the active count on the host: not inside a graph
         // capture (the library's own plan, or a caller capturing this stream)
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cap = cudaStreamCaptureStatusNone;
         const bool can_poll = sp.tol2 > 0.0 && !staging && cap == cudaStreamCaptureStatusNone;
         int poll_slot = 0, poll_prev = -1;
         for (int it = 0; it <= max_iter; ++it) {
