@@ -17,14 +17,15 @@
 // shared memory by the warps that later drain the accumulators (FP32 atomics, 32
 // consecutive input channels per instruction).  Pixel rows are split over CTAs.
 //
-// What bounds it: the issuing warp (about 500 cycles per stage for its wait and
-// commit, 35 to 48 per MMA) next to the MMA rate (M=128, N=192: 96 cycles; N=96: 56),
-// and at one image the drain, 10 us of atomics.
+// What bounds it: HBM in the 32 -> 32 layer (273 MB in 59 us, 0.68 of the copy rate);
+// elsewhere the issuing warp (about 500 cycles per stage for its wait and commit, 35
+// to 48 per MMA) next to the MMA rate (M=128, N=192: 96 cycles; N=96: 56), and at one
+// image the drain, 10 us of atomics.
 // Against copies of both operands in a channel-major layout (x three times, shifted
 // by kx), one tap per CTA, and a kernel for the bias, 32 images: 32 -> 32 at
-// 256 x 256 448 -> 191 us, 96 -> 32 790 -> 195, 192 -> 64 at 128 x 128 396 -> 99,
-// 384 -> 128 at 64 x 64 237 -> 104, 256 -> 256 at 32 x 32 113 -> 47; the training
-// step 5.98 -> 3.60 ms.  One row per stage with a barrier per operand and ring:
+// 256 x 256 448 -> 57 us, 96 -> 32 790 -> 156, 192 -> 64 at 128 x 128 396 -> 98,
+// 384 -> 128 at 64 x 64 237 -> 104, 256 -> 256 at 32 x 32 113 -> 46; the training
+// step 5.98 -> 3.26 ms.  One row per stage with a barrier per operand and ring:
 // 384 -> 128 149, 256 -> 256 83.
 #include "synk_internal.cuh"
 #include "umma.cuh"

@@ -13,8 +13,8 @@
 // gather takes at least four cycles, measured 4.06), so a step's two 16-byte
 // gathers take 2.03 cycles per slice, while the shared index and weight
 // arithmetic takes about 1.1; one slice at a time took 2.6-3.2 issue cycles.
-// N=512, 360 angles: 16 slices x 10 iterations 18.6 -> 9.2 ms, 512 slices
-// 105.7 -> 50.0 us per slice and iteration.
+// N=512, 360 angles: 16 slices x 10 iterations 18.6 -> 8.95 ms, 512 slices
+// 105.7 -> 49.7 us per slice and iteration.
 #include <math.h>
 
 #include "synk_internal.cuh"
