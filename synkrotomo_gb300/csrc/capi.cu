@@ -18,6 +18,7 @@
 #include "bp_tile.cuh"
 #include "umma_gemm.cuh"
 #include "unet.cuh"
+#include "poll_word.cuh"
 
 using namespace synk;
 
@@ -34,7 +35,8 @@ struct synk_context {
     cudaStream_t stream = nullptr;
     std::string err;
     int *d_status = nullptr;   // written by kernels whose waits ran out (SYNK_ETIMEOUT)
-    int *h_poll = nullptr;     // pinned: active-slice counts read back by the SIRT loop's stopping rule
+    unsigned long long *h_poll = nullptr;   // pinned: active-slice counts read back by the SIRT loop's stopping rule (poll_done)
+    int poll_calls = 0;        // number of the call that a count belongs to
     cudaEvent_t poll_ev[2] = {nullptr, nullptr};
     unsigned long long barrier_timeout_ns = 2000000000ull;
     unsigned barrier_extra = 0;   // fault injection: blocks a grid barrier waits for that never come
@@ -531,10 +533,11 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
     for (int i = 0; i < nprob; ++i) sorted[i] = host[order[i]];
     SirtProblem *dprobs;
     long long *totals;
+    constexpr int kWords = 10;   // barrier 0-1, work counters 4-6, the stopping rule's call and count 8-9
     unsigned *words;
     SYNK_CUDA(sc.get(&dprobs, (size_t)nprob), "cudaMallocAsync(problem table)");
     SYNK_CUDA(sc.get(&totals, 2), "cudaMallocAsync");
-    SYNK_CUDA(sc.get(&words, 8), "cudaMallocAsync");
+    SYNK_CUDA(sc.get(&words, kWords), "cudaMallocAsync");
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cap = cudaStreamCaptureStatusNone;
     if (staging) {
@@ -553,7 +556,7 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         SYNK_CUDA(cudaMemcpyAsync(dprobs, sorted.data(), sizeof(SirtProblem) * nprob, cudaMemcpyHostToDevice, st),
                   "upload problem table");
     }
-    SYNK_CUDA(cudaMemsetAsync(words, 0, sizeof(unsigned) * 8, st), "memset");
+    SYNK_CUDA(cudaMemsetAsync(words, 0, sizeof(unsigned) * kWords, st), "memset");
     SYNK_CUDA(launch_sirt_plan(dprobs, nprob, totals, st), "plan kernel");
     SirtParams sp;
     sp.probs = dprobs;
@@ -584,11 +587,16 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
         SYNK_CUDA(launch_sirt_small(ss, small_grid, st), "small SIRT kernel");
     } else if (split) {
         sp.dynamic = 0;
-        int *active = reinterpret_cast<int *>(words + 7);
+        int *call = reinterpret_cast<int *>(words + 8), *active = call + 1;    // poll_done's word
         // the early exit reads the active count on the host: not inside a graph
         // capture (the library's own plan, or a caller capturing this stream)
         const bool can_poll = sp.tol2 > 0.0 && !staging && cap == cudaStreamCaptureStatusNone;
         int poll_slot = 0, poll_prev = -1;
+        if (can_poll) {
+            ctx->poll_calls = ctx->poll_calls == INT_MAX ? 1 : ctx->poll_calls + 1;
+            fill_i32_kernel<<<1, 1, 0, st>>>(call, 1, ctx->poll_calls);
+            SYNK_CUDA(cudaGetLastError(), "fill kernel");
+        }
         for (int it = 0; it <= max_iter; ++it) {
             if (slices)
                 SYNK_CUDA(launch_sirt_fp_slices(host[0], it, sp.tol2, sp.record_final, sp.tol2 > 0.0 || want_res, st),
@@ -609,12 +617,13 @@ int sirt_batch(synk_context *ctx, int nprob, const synk_sirt_problem *in, double
             // the stream at each check cost more than stopping saved (N=128:
             // 184 iterations to the residual 4.20 ms, 200 iterations 3.96 ms).
             if (can_poll && (it & 15) == 15) {
-                SYNK_CUDA(cudaMemcpyAsync(ctx->h_poll + poll_slot, active, sizeof(int), cudaMemcpyDeviceToHost, st),
+                SYNK_CUDA(cudaMemcpyAsync(ctx->h_poll + poll_slot, call, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                          st),
                           "read active");
                 SYNK_CUDA(cudaEventRecord(ctx->poll_ev[poll_slot], st), "record poll");
                 if (poll_prev >= 0) {
                     SYNK_CUDA(cudaEventSynchronize(ctx->poll_ev[poll_prev]), "wait poll");
-                    if (ctx->h_poll[poll_prev] == 0) break;
+                    if (poll_done(*(volatile unsigned long long *)(ctx->h_poll + poll_prev), ctx->poll_calls)) break;
                 }
                 poll_prev = poll_slot;
                 poll_slot ^= 1;
@@ -680,7 +689,7 @@ int synk_context_new(synk_context **out, int device, void *stream) {
     ctx->stream = static_cast<cudaStream_t>(stream);
     if (cudaMalloc(&ctx->d_status, sizeof(int)) != cudaSuccess ||
         cudaMemset(ctx->d_status, 0, sizeof(int)) != cudaSuccess ||
-        cudaHostAlloc(&ctx->h_poll, 2 * sizeof(int), cudaHostAllocDefault) != cudaSuccess ||
+        cudaHostAlloc(&ctx->h_poll, 2 * sizeof(unsigned long long), cudaHostAllocDefault) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->poll_ev[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->poll_ev[1], cudaEventDisableTiming) != cudaSuccess) {
         synk_context_free(ctx);
